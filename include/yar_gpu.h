@@ -379,13 +379,19 @@ typedef struct yar_gpu_options {
                                        the traversal kernel is chosen; UINT32_MAX: never */
 } yar_gpu_options;
 
-/* Traversal kernels (identical results, different speed): persistent warps
+/* Traversal kernels (identical results, different speed).  With AUTO, a scene
+ * whose objects are at most translated is cast through an 8-wide tree that the
+ * upload builds; every hit is settled against the kd-tree, and rays it does not
+ * settle walk the kd-tree one per thread (renders of scenes of tessellated
+ * axis-parallel planes walk it for every ray): both are reported as PER_RAY.
+ * The others, fixed by the options or chosen for scenes with rotated or scaled
+ * objects, walk the kd-tree: persistent warps
  * at high occupancy (PERSISTENT_64: a register cap for 8 blocks of 128
  * threads per SM, 64 registers, for closest-hit rays and for 12 blocks, 40
  * registers, for any-hit rays), persistent warps with up to 128 registers
- * (PERSISTENT_128), or one ray per thread.  With AUTO the first large enough
- * batch of each ray kind (and each render bounce) after a scene upload times
- * all three and keeps the fastest. */
+ * (PERSISTENT_128), or one ray per thread.  In those scenes AUTO times, on the
+ * first large enough batch of each ray kind (and each render bounce) after the
+ * scene upload, all of them and keeps the fastest. */
 #define YAR_TRAVERSAL_AUTO 0
 #define YAR_TRAVERSAL_PERSISTENT_64 1
 #define YAR_TRAVERSAL_PERSISTENT_128 2
@@ -489,7 +495,7 @@ typedef struct yar_batch_scene_stats {
     double variance;              /* render_scene's variance_estimate */
     float completion_seconds;     /* batch start to this scene's resolved film, GPU clock */
     uint64_t paths;               /* camera paths */
-    uint32_t traversal_kernel[2]; /* YAR_TRAVERSAL_* used for closest-hit and any-hit rays */
+    uint32_t traversal_kernel[2]; /* YAR_TRAVERSAL_* used for closest-hit and any-hit rays (as yar_gpu_traversal_kernels) */
 } yar_batch_scene_stats;
 
 typedef struct yar_batch_stats {

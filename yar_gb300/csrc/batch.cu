@@ -221,9 +221,11 @@ cudaError_t enqueue_scene(Batch& bt, int si, bool one_spp, unsigned long long* s
             a.count = ctr + 7;
             a.n_max = paths;
             a.next_ray = ctr + 4;
+            a.next_ray_zeroed = true;
             a.err = reinterpret_cast<int*>(ctr + 3);
             a.hit4 = q.ext_hit4;
             a.hit2 = q.ext_hit2;
+            a.answers = q.shd_slot;  // the shade kernel fills it later
             e = launch_extend(sub->ds, a, sc.kernel[0], st);
             if (e != cudaSuccess) break;
             if (mixed) {
@@ -241,8 +243,10 @@ cudaError_t enqueue_scene(Batch& bt, int si, bool one_spp, unsigned long long* s
             sh.n_max = paths;
             sh.perm = q.shd_slot;
             sh.next_ray = ctr + 5;
+            sh.next_ray_zeroed = true;
             sh.err = reinterpret_cast<int*>(ctr + 3);
             sh.occluded = ps.occluded;
+            sh.answers = reinterpret_cast<uint32_t*>(q.ext_hit2);  // the shade kernel has read it
             e = launch_shadow(sub->ds, sh, sc.kernel[1], st);
             if (e != cudaSuccess) break;
             Cast_Args pr;
@@ -251,9 +255,11 @@ cudaError_t enqueue_scene(Batch& bt, int si, bool one_spp, unsigned long long* s
             pr.n_max = paths;
             pr.perm = q.prb_slot;
             pr.next_ray = ctr + 6;
+            pr.next_ray_zeroed = true;
             pr.err = reinterpret_cast<int*>(ctr + 3);
             pr.hit4 = ps.probe_hit4;
             pr.hit2 = ps.probe_hit2;
+            pr.answers = reinterpret_cast<uint32_t*>(q.ext_hit2);
             e = launch_extend(sub->ds, pr, sc.kernel[0], st);
             if (e != cudaSuccess) break;
             connect_kernel<<<kFixedGrid, kBlock, 0, st>>>(p, S, q.ext_slot[cur], paths, ps, nullptr, ctr + 7);
@@ -396,8 +402,8 @@ int render_batch(yar_gpu_ctx* ctx, const yar_flat_scene* const* scenes, uint32_t
             a.hit4 = dp<float4>(hits);
             a.hit2 = reinterpret_cast<uint2*>(dp<float4>(hits) + n);
             for (int kind = 0; kind < 2 && e == cudaSuccess; kind++) {
-                if (s.sub->forced_kernel >= 0) {
-                    s.kernel[kind] = s.sub->forced_kernel;
+                if (s.sub->cast_kernel[kind] >= 0) {  // fixed by the options, or the wide tree
+                    s.kernel[kind] = s.sub->cast_kernel[kind];
                     continue;
                 }
                 Cast_Args k = a;
@@ -472,8 +478,10 @@ int render_batch(yar_gpu_ctx* ctx, const yar_flat_scene* const* scenes, uint32_t
             scene_stats[i].variance = var;
             scene_stats[i].completion_seconds = (float)((double)(st[1 + i] - st[0]) * 1e-9);
             scene_stats[i].paths = s.samples;
-            scene_stats[i].traversal_kernel[0] = (uint32_t)s.kernel[0] + YAR_TRAVERSAL_PERSISTENT_64;
-            scene_stats[i].traversal_kernel[1] = (uint32_t)s.kernel[1] + YAR_TRAVERSAL_PERSISTENT_64;
+            for (int kind = 0; kind < 2; kind++)
+                scene_stats[i].traversal_kernel[kind] = s.kernel[kind] == kCastWide
+                                                            ? (uint32_t)YAR_TRAVERSAL_PER_RAY
+                                                            : (uint32_t)s.kernel[kind] + YAR_TRAVERSAL_PERSISTENT_64;
         }
     }
     if (e != cudaSuccess) return cuda_fail(ctx, e, "render batch: results");

@@ -11,7 +11,9 @@
 // The same kernels serve the C-ABI casts (results as structure of arrays at
 // the ray's index) and the render wavefront (hit records at the path slot).
 #include "context.hpp"
+#include "wide_bvh.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <type_traits>
 
@@ -53,7 +55,7 @@ __global__ void __launch_bounds__(kCastBlock, MINB) cast_persistent(Device_Scene
     const uint32_t n = a.count ? *a.count : a.n;
     Traversal<ANY> tr;
     __shared__ uint2 stack_smem[SHORT > 0 ? SHORT * kCastBlock : 1];
-    typename std::conditional<(SHORT > 0), Split_Stack<SHORT, kCastBlock>, Local_Stack>::type stack;
+    typename std::conditional<(SHORT > 0), Split_Stack<SHORT, kCastBlock, kStackEntries>, Local_Stack>::type stack;
     if constexpr (SHORT > 0) stack.smem = stack_smem + threadIdx.x;
     bool have = false, alive = true;
     uint32_t batch_next = 0, batch_end = 0;  // warp-uniform
@@ -177,6 +179,163 @@ __global__ void __launch_bounds__(kCastBlock) cast_per_ray_vote(Device_Scene s, 
     }
 }
 
+// The wide tree's two kernels.
+//
+// cast_wide: persistent warps whose lanes each own a ray, one mode (visit a
+// node, test a leaf child) per warp iteration.  Lanes whose ray is done wait
+// until kWideRefill of them are, then write their results (a miss is final, a
+// hit leaves its answer for the second kernel) and take new rays.  Bound by
+// issue (78% of the cycles on 16M random rays in 2.4M triangles, 17 of 32 lanes
+// in an instruction, about 200 warp instructions per ray against the kd-tree
+// kernel's 880); measured there, closest / any hit: 8 blocks of 128 threads per
+// SM 4.4 / 3.2 ms, 6 blocks 4.6 / 3.5; refills at 4, 8, 12, 16, 20 done lanes
+// 5.1, 4.81, 4.78, 5.2, 5.5 ms (before the entries below); tests as soon as
+// half as many lanes wait for one as visit 4.8 ms, when more do 5.0.
+//
+// settle_wide: every hit against the kd-tree, with full warps.  A settled hit
+// costs dependent loads; inside the first kernel (at its registers, with the
+// lanes that happen to be done) they took as long as the traversal: 7.9 ms
+// together, 5.7 as two kernels, 4.4 once the descents begin at the triangles'
+// entries.  Now bound by scattered DRAM reads (about 4 TB/s).
+constexpr int kWideShortStack = 10;  // shared-memory entries; deeper ones in local memory
+constexpr int kWideRefill = 12;
+constexpr int kWideBlocks = 8, kSettleBlocks = 8;
+
+template <bool ANY>
+__device__ __forceinline__ void write_settled(int status, const Hit& h, uint32_t ray, const Cast_Args& a) {
+    const uint32_t i = a.perm ? __ldg(a.perm + ray) : ray;
+    if (status < 0) atomicOr(a.err, 1);
+    if (ANY) {
+        a.occluded[i] = (uint8_t)(status > 0 ? 1 : 0);
+        return;
+    }
+    const bool hit = status > 0;
+    if (a.hit4) {  // render layout
+        a.hit4[i] = make_float4(h.t, h.b0, h.b1, h.b2);
+        a.hit2[i] = hit ? make_uint2(h.prim, h.object) : make_uint2(0xffffffffu, 0xffffffffu);
+        return;
+    }
+    if (a.t) a.t[i] = status < 0 ? __ldg(a.rays + 2 * (size_t)ray).w : h.t;
+    if (a.prim) a.prim[i] = hit ? h.prim : 0xffffffffu;
+    if (a.object) a.object[i] = hit ? h.object : 0xffffffffu;
+    if (a.bary) a.bary[i] = hit ? make_float2(h.b1, h.b2) : make_float2(0.f, 0.f);
+}
+
+template <bool ANY>
+__global__ void __launch_bounds__(kCastBlock, kWideBlocks)
+cast_wide(const __grid_constant__ Device_Scene s, const __grid_constant__ Cast_Args a) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned lower = (1u << lane) - 1u;
+    const uint32_t n = a.count ? *a.count : a.n;
+    // rays a warp takes per atomic: its share of a short queue, so that few
+    // rays spread over the chip; at most kBatch
+    const uint32_t batch = min(kBatch, n / (gridDim.x * (kCastBlock / 32)) + 1u);
+    __shared__ uint2 stack_smem[kWideShortStack * kCastBlock];
+    Split_Stack<kWideShortStack, kCastBlock, kWideStackSize> stack;
+    stack.smem = stack_smem + threadIdx.x;
+    Wide_Traversal<ANY> w;
+    enum { kEmpty, kActive, kFinished };
+    int state = kEmpty;
+    bool more = true;                            // warp-uniform: the queue may hold further rays
+    uint32_t batch_next = 0, batch_end = 0;      // warp-uniform
+    for (;;) {
+        const unsigned active = __ballot_sync(full, state == kActive);
+        if (__popc(active) <= 32 - kWideRefill && (more || !active)) {
+            if (state == kFinished) {
+                a.answers[w.ray] = w.best == kWideNone ? kWideNone : w.answer();
+                if (w.best == kWideNone) {
+                    Hit h;
+                    h.t = ANY ? 0.f : w.t;
+                    h.prim = h.object = 0xffffffffu;
+                    h.b0 = h.b1 = h.b2 = 0.f;
+                    write_settled<ANY>(0, h, w.ray, a);
+                }
+                state = kEmpty;
+            }
+            while (more) {
+                const unsigned want = __ballot_sync(full, state == kEmpty);
+                if (!want) break;
+                if (batch_next >= batch_end) {
+                    uint32_t b = 0;
+                    if (lane == 0) b = atomicAdd(a.next_ray, batch);
+                    b = __shfl_sync(full, b, 0);
+                    if (b >= n) {
+                        more = false;
+                        break;
+                    }
+                    batch_next = b;
+                    batch_end = min(b + batch, n);
+                }
+                const uint32_t avail = batch_end - batch_next;
+                const uint32_t rank = (uint32_t)__popc(want & lower);
+                if (state == kEmpty && rank < avail) {
+                    const uint32_t ray = batch_next + rank;
+                    const float4 r0 = __ldg(a.rays + 2 * (size_t)ray), r1 = __ldg(a.rays + 2 * (size_t)ray + 1);
+                    if (w.begin(s, ray, make_float3(r0.x, r0.y, r0.z), make_float3(r1.x, r1.y, r1.z), r0.w))
+                        state = kActive;
+                    else  // outside the numbers the wide tree covers
+                        a.answers[ray] = kWideWalk;
+                }
+                batch_next += min((uint32_t)__popc(want), avail);
+            }
+            if (!__ballot_sync(full, state == kActive)) break;
+        }
+        const unsigned testing = __ballot_sync(full, state == kActive && w.pending());
+        const unsigned visiting = __ballot_sync(full, state == kActive && !w.pending());
+        if (2 * __popc(testing) > __popc(visiting)) {
+            if (state == kActive && w.pending()) {
+                if (w.test(s)) state = kFinished;
+                else if (!w.pending() && !w.next_group(stack)) state = kFinished;
+            }
+        } else {
+            if (state == kActive && !w.pending()) {
+                w.visit(s, stack);
+                if (!w.pending() && !w.next_group(stack)) state = kFinished;
+            }
+        }
+    }
+}
+
+// The hits of a warp's rays are listed in shared memory and settled 32 at a
+// time (less than half of a batch's rays may hit).
+template <bool ANY>
+__global__ void __launch_bounds__(kCastBlock, kSettleBlocks)
+settle_wide(const __grid_constant__ Device_Scene s, const __grid_constant__ Cast_Args a) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned lower = (1u << lane) - 1u;
+    const uint32_t n = a.count ? *a.count : a.n;
+    __shared__ uint2 list_smem[kCastBlock / 32][64];
+    uint2* list = list_smem[threadIdx.x >> 5];
+    uint32_t listed = 0;  // warp-uniform
+    uint64_t base = ((uint64_t)blockIdx.x * kCastBlock + threadIdx.x) & ~31ull;
+    for (;;) {
+        const bool last = base >= n;
+        if (!last) {
+            const uint32_t ray = (uint32_t)base + lane;
+            const uint32_t answer = base + lane < n ? a.answers[ray] : kWideNone;
+            const unsigned hits = __ballot_sync(full, answer != kWideNone);
+            if (answer != kWideNone) list[listed + __popc(hits & lower)] = make_uint2(ray, answer);
+            listed += __popc(hits);
+            __syncwarp();
+            base += (uint64_t)gridDim.x * kCastBlock;
+        }
+        if (listed >= 32u || (last && listed)) {
+            const uint32_t k = min(listed, 32u);
+            listed -= k;
+            if ((uint32_t)lane < k) {
+                const uint2 entry = list[listed + lane];
+                Hit h;
+                const int status = wide_settle<ANY>(s, a.rays, entry.x, entry.y, h);
+                write_settled<ANY>(status, h, entry.x, a);
+            }
+            __syncwarp();
+        }
+        if (last && !listed) break;
+    }
+}
+
 // Persistent launch shape, measured on GB300 with the 2.42M-triangle ray-cast
 // workload (16M + 16M incoherent rays).  With one mode per warp iteration,
 // one node fetch per descent step: closest hit 19.8 ms against 21.3 ms at two
@@ -229,14 +388,24 @@ cudaError_t launch(const Device_Scene& s, const Cast_Args& a, int kernel, cudaSt
         const uint32_t bound = a.count ? a.n_max : a.n;
         if (bound == 0) return cudaSuccess;
         if (kernel == kCastPerRay)
-            cast_per_ray<ANY><<<(bound + kCastBlock - 1) / kCastBlock, kCastBlock, 0, stream>>>(s, a);
+            // queues sized on the device: at most 64 blocks per SM (a queue bound of 16M rays is
+            // 131,072 blocks, 25 us of launch for the deep bounces' nearly empty queues)
+            cast_per_ray<ANY><<<std::min<uint32_t>((bound + kCastBlock - 1) / kCastBlock, a.count ? 152u * 64u : 0xffffffffu),
+                                kCastBlock, 0, stream>>>(s, a);
         else
             cast_per_ray_vote<ANY><<<(bound + kCastBlock - 1) / kCastBlock, kCastBlock, 0, stream>>>(s, a);
         return cudaGetLastError();
     }
-    cudaError_t e = cudaMemsetAsync(a.next_ray, 0, sizeof(uint32_t), stream);
+    cudaError_t e = a.next_ray_zeroed ? cudaSuccess : cudaMemsetAsync(a.next_ray, 0, sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
-    if (kernel == kCastPersistent128) {
+    if (kernel == kCastWide) {
+        static std::atomic<int> grid[kMaxDevices], settle_grid[kMaxDevices];
+        cast_wide<ANY><<<resident_grid(cast_wide<ANY>, grid), kCastBlock, 0, stream>>>(s, a);
+        const uint32_t bound = a.count ? a.n_max : a.n;
+        const uint32_t blocks = std::min<uint32_t>((bound + kCastBlock - 1) / kCastBlock,
+                                                   (uint32_t)resident_grid(settle_wide<ANY>, settle_grid));
+        settle_wide<ANY><<<std::max(1u, blocks), kCastBlock, 0, stream>>>(s, a);
+    } else if (kernel == kCastPersistent128) {
         static std::atomic<int> grid[kMaxDevices];
         auto k = cast_persistent<ANY, 4, kWhileWhile, kSharedStackEntries>;
         k<<<resident_grid(k, grid), kCastBlock, 0, stream>>>(s, a);

@@ -81,12 +81,15 @@ struct yar_gpu_ctx {
     // scene
     bool has_scene = false;
     yar::Device_Buffer scene_nodes, mesh_nodes, objects, tris;
+    yar::Device_Buffer wide_nodes, wide_tris, wide_entries;  // wide_bvh.cuh
+    bool wide_planar = false;  // most of the scene's triangles tessellate axis-parallel planes
     yar::Device_Scene ds;
     yar::Render_Scene render;
 
     // staging area for host-buffer casts
     uint32_t staging_capacity = 0;
     yar::Device_Buffer d_rays, d_t, d_prim, d_obj, d_bary, d_occ;
+    yar::Device_Buffer d_answers;  // the wide tree's answers of a cast
     int* d_error = nullptr;  // device error word (stack overflow, bounded-wait expiry)
     uint32_t* d_counter = nullptr;  // ray hand-out counters of the persistent cast kernels, one per pipeline chunk
     // host-buffer casts in chunks: copies in, the traversal on two compute
@@ -145,6 +148,7 @@ struct Cast_Args {
     uint32_t n_max = 0;               // upper bound of *count (grid of the one-ray-per-thread kernel)
     const uint32_t* perm = nullptr;   // output index of each ray position (null: the position)
     uint32_t* next_ray = nullptr;     // one device word used to hand out rays (zeroed per launch)
+    bool next_ray_zeroed = false;     // the caller has zeroed it
     int* err = nullptr;               // error word (traversal-stack overflow)
     // closest hit, C-ABI layout (any pointer may be null)
     float* t = nullptr;
@@ -156,6 +160,8 @@ struct Cast_Args {
     uint2* hit2 = nullptr;
     // any hit
     uint8_t* occluded = nullptr;
+    // the wide tree's answers, one word per ray position (kCastWide)
+    uint32_t* answers = nullptr;
 };
 // Traversal kernels: persistent warps at high occupancy (closest hit 10
 // blocks per SM, any hit 12 blocks), persistent
@@ -167,8 +173,16 @@ enum Cast_Kernel {
     kCastPersistent128 = 1,
     kCastPerRay = 2,
     kCastPerRayVote = 3,  // one ray per thread, one mode per warp iteration
-    kCastKernelCount = 4
+    kCastKernelCount = 4,
+    // the wide tree first, the kd-tree settles (wide_bvh.cuh): every cast of a
+    // scene that has a wide tree, unless the options fix one of the others
+    kCastWide = 4
 };
+// The wide tree of the uploaded scene (wide_build.cu): built into ctx->ds, or
+// left out (ctx->ds.wide_nodes null) where the scene does not allow one.
+cudaError_t wide_build(yar_gpu_ctx* ctx, const yar_flat_scene* scene, const uint32_t* tri_offset,
+                       const uint32_t* node_offset);
+void wide_release(yar_gpu_ctx* ctx);
 cudaError_t launch_extend(const Device_Scene& s, const Cast_Args& a, int kernel, cudaStream_t stream);
 cudaError_t launch_shadow(const Device_Scene& s, const Cast_Args& a, int kernel, cudaStream_t stream);
 // Runs the batch once untimed and three times with each kernel (event-timed

@@ -53,6 +53,12 @@ struct Device_Scene {
     const uint4* texture_mips = nullptr;
     float scene_bounds[6] = {0, 0, 0, 0, 0, 0};
     uint32_t object_count = 0;
+    // the wide tree over the scene's triangles (wide_bvh.cuh); null without one
+    const uint4* wide_nodes = nullptr;
+    const float4* wide_tris = nullptr;
+    const float4* wide_entries = nullptr;  // per primitive (triangle of an object): in its mesh's tree, in the scene's
+    float wide_reach = 0.f;   // largest coordinate of its triangles, before and after their translation
+    uint32_t wide_flags = 0;  // some triangle has an alpha test or casts no shadow
 };
 
 struct Hit {
@@ -132,23 +138,18 @@ __device__ __forceinline__ Watertight_Ray watertight_setup(float3 d, float3 inv)
     return w;
 }
 
-// intersect_triangle_watertight, src/ref/intersection.cpp:64-113.
+// intersect_triangle_watertight, src/ref/intersection.cpp:64-113, from the
+// vertices relative to the ray origin, components in the order kx, ky, kz.
 // Returns +inf when there is no intersection.
-__device__ __forceinline__ float watertight(float3 o, const Watertight_Ray& w, float4 v0, float4 v1, float4 v2,
-                                            float& b0, float& b1, float& b2) {
-    const float ox = sel3(o.x, o.y, o.z, w.kx), oy = sel3(o.x, o.y, o.z, w.ky), oz = sel3(o.x, o.y, o.z, w.kz);
-    const float p0x = sel3(v0.x, v0.y, v0.z, w.kx) - ox, p0y = sel3(v0.x, v0.y, v0.z, w.ky) - oy,
-                p0z = sel3(v0.x, v0.y, v0.z, w.kz) - oz;
-    const float p1x = sel3(v1.x, v1.y, v1.z, w.kx) - ox, p1y = sel3(v1.x, v1.y, v1.z, w.ky) - oy,
-                p1z = sel3(v1.x, v1.y, v1.z, w.kz) - oz;
-    const float p2x = sel3(v2.x, v2.y, v2.z, w.kx) - ox, p2y = sel3(v2.x, v2.y, v2.z, w.ky) - oy,
-                p2z = sel3(v2.x, v2.y, v2.z, w.kz) - oz;
-    const float x0 = p0x + w.sx * p0z;
-    const float y0 = p0y + w.sy * p0z;
-    const float x1 = p1x + w.sx * p1z;
-    const float y1 = p1y + w.sy * p1z;
-    const float x2 = p2x + w.sx * p2z;
-    const float y2 = p2y + w.sy * p2z;
+__device__ __forceinline__ float watertight_edges(float p0x, float p0y, float p0z, float p1x, float p1y, float p1z,
+                                                  float p2x, float p2y, float p2z, float sx, float sy, float sz,
+                                                  float& b0, float& b1, float& b2) {
+    const float x0 = p0x + sx * p0z;
+    const float y0 = p0y + sy * p0z;
+    const float x1 = p1x + sx * p1z;
+    const float y1 = p1y + sy * p1z;
+    const float x2 = p2x + sx * p2z;
+    const float y2 = p2y + sy * p2z;
     float e0 = x1 * y2 - y1 * x2;
     float e1 = x2 * y0 - y2 * x0;
     float e2 = x0 * y1 - y0 * x1;
@@ -161,9 +162,9 @@ __device__ __forceinline__ float watertight(float3 o, const Watertight_Ray& w, f
     if ((e0 < 0.f || e1 < 0.f || e2 < 0.f) && (e0 > 0.f || e1 > 0.f || e2 > 0.f)) return inf;
     const float det = e0 + e1 + e2;
     if (det == 0.f) return inf;
-    const float z0 = w.sz * p0z;
-    const float z1 = w.sz * p1z;
-    const float z2 = w.sz * p2z;
+    const float z0 = sz * p0z;
+    const float z1 = sz * p1z;
+    const float z2 = sz * p2z;
     const float t_scaled = e0 * z0 + e1 * z1 + e2 * z2;
     if ((__float_as_uint(det) ^ __float_as_uint(t_scaled)) >> 31) return inf;
     const float inv_det = 1.f / det;
@@ -172,6 +173,16 @@ __device__ __forceinline__ float watertight(float3 o, const Watertight_Ray& w, f
     b1 = e1 * inv_det;
     b2 = e2 * inv_det;
     return t;
+}
+
+__device__ __forceinline__ float watertight(float3 o, const Watertight_Ray& w, float4 v0, float4 v1, float4 v2,
+                                            float& b0, float& b1, float& b2) {
+    const float ox = sel3(o.x, o.y, o.z, w.kx), oy = sel3(o.x, o.y, o.z, w.ky), oz = sel3(o.x, o.y, o.z, w.kz);
+    return watertight_edges(sel3(v0.x, v0.y, v0.z, w.kx) - ox, sel3(v0.x, v0.y, v0.z, w.ky) - oy,
+                            sel3(v0.x, v0.y, v0.z, w.kz) - oz, sel3(v1.x, v1.y, v1.z, w.kx) - ox,
+                            sel3(v1.x, v1.y, v1.z, w.ky) - oy, sel3(v1.x, v1.y, v1.z, w.kz) - oz,
+                            sel3(v2.x, v2.y, v2.z, w.kx) - ox, sel3(v2.x, v2.y, v2.z, w.ky) - oy,
+                            sel3(v2.x, v2.y, v2.z, w.kz) - oz, w.sx, w.sy, w.sz, b0, b1, b2);
 }
 
 // The alpha test of both leaf callbacks (src/ref/kdtree.cpp:31-38, :69-77):
@@ -514,10 +525,10 @@ struct Local_Stack {
 // Traversal stack whose first SHORT entries live in shared memory, laid out
 // entry-major ([entry][thread], conflict-free for a warp), with the rarely
 // used deeper entries in local memory.
-template <int SHORT, int BLOCK>
+template <int SHORT, int BLOCK, int ENTRIES>
 struct Split_Stack {
     uint2* smem;  // this thread's column: base + threadIdx.x
-    uint2 deep[kStackEntries - SHORT];
+    uint2 deep[ENTRIES - SHORT];
     __device__ __forceinline__ void push(int sp, uint32_t node, float t_max) {
         const uint2 v = make_uint2(node, __float_as_uint(t_max));
         if (sp < SHORT) smem[sp * BLOCK] = v;

@@ -651,6 +651,7 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
                                                                     q.ext_rays[from ^ 1], q.ext_slot[from ^ 1],
                                                                     ray_keys, ray_hist, count_dev, count);
     };
+    const uint32_t settles = ctx->ds.wide_nodes ? 3u : 0u;  // the wide tree's casts are two kernels each
     // The bounce loop over extend queue 0 of `count` paths; bounce0 picks the
     // traversal kernels.  Sets e; returns a YAR_ERR_* for a traversal overflow.
     auto run_bounces = [&](const Render_Params& pp, uint32_t count, int bounce0) -> int {
@@ -683,7 +684,7 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
             e = trace_light_queues(ctx, q, ps, count, bounce, st);
             if (e != cudaSuccess) break;
             connect_kernel<<<grid_for(count), kBlock, 0, st>>>(pp, S, q.ext_slot[cur], count, ps, nullptr);
-            launches += mixed ? 7 : 5;
+            launches += (mixed ? 7 : 5) + settles;
             uint32_t h[4];
             e = cudaMemcpyAsync(h, q.counters, sizeof(h), cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -698,13 +699,14 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
     };
     // The same bounces with the queue lengths on the device: every iteration
     // runs (the kernels exit on an empty queue); first_paths = 0 takes the
-    // first count from counters[0] (a tail wave's queue).
-    auto run_bounces_device = [&](const Render_Params& pp, uint32_t first_paths, uint32_t max_paths, int bounce0) {
+    // first count from counters[0] (a tail wave's queue, whose paths have
+    // `behind` vertices behind them).
+    auto run_bounces_device = [&](const Render_Params& pp, uint32_t first_paths, uint32_t max_paths, int bounce0, int behind) {
         Queues qd = qo;
         qd.ext_count = q.counters + 7;
         const int grid = grid_for(max_paths);
         int cur = 0;
-        for (int it = 0; it <= p.max_bounces + 1 && e == cudaSuccess; it++) {
+        for (int it = 0; it <= p.max_bounces + 1 - behind && e == cudaSuccess; it++) {
             const int bounce = bounce0 + it;
             bounce_begin_kernel<<<1, 1, 0, st>>>(q.counters, it == 0 ? first_paths : 0u, rays_dev);
             if (sort_rays && it > 0) {
@@ -717,9 +719,11 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
             a.count = q.counters + 7;
             a.n_max = max_paths;
             a.next_ray = q.counters + 4;
+            a.next_ray_zeroed = true;
             a.err = reinterpret_cast<int*>(q.counters + 3);
             a.hit4 = q.ext_hit4;
             a.hit2 = q.ext_hit2;
+            a.answers = q.shd_slot;  // the shade kernel fills it later
             e = launch_extend(ctx->ds, a, render_choice(ctx, 0, bounce), st);
             if (e != cudaSuccess) break;
             order_queue(qd, max_paths, grid);
@@ -731,8 +735,10 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
             sh.n_max = max_paths;
             sh.perm = q.shd_slot;
             sh.next_ray = q.counters + 5;
+            sh.next_ray_zeroed = true;
             sh.err = reinterpret_cast<int*>(q.counters + 3);
             sh.occluded = ps.occluded;
+            sh.answers = reinterpret_cast<uint32_t*>(q.ext_hit2);  // the shade kernel has read it
             e = launch_shadow(ctx->ds, sh, render_choice(ctx, 1, bounce), st);
             if (e != cudaSuccess) break;
             Cast_Args pr;
@@ -741,13 +747,15 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
             pr.n_max = max_paths;
             pr.perm = q.prb_slot;
             pr.next_ray = q.counters + 6;
+            pr.next_ray_zeroed = true;
             pr.err = reinterpret_cast<int*>(q.counters + 3);
             pr.hit4 = ps.probe_hit4;
             pr.hit2 = ps.probe_hit2;
+            pr.answers = reinterpret_cast<uint32_t*>(q.ext_hit2);
             e = launch_extend(ctx->ds, pr, render_choice(ctx, 0, bounce), st);
             if (e != cudaSuccess) break;
             connect_kernel<<<grid, kBlock, 0, st>>>(pp, S, q.ext_slot[cur], max_paths, ps, nullptr, q.counters + 7);
-            launches += mixed ? 8 : 6;
+            launches += (mixed ? 8 : 6) + settles;
             cur ^= 1;
         }
         bounce_begin_kernel<<<1, 1, 0, st>>>(q.counters, 0u, rays_dev);  // adds the last bounce's rays
@@ -761,7 +769,7 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
         launch_generate(p, (uint32_t)first, cp, dptr<float>(B[2]), dptr<float>(B[3]), image_samples, ps, q, st);
         launches++;
         if (device_driven) {
-            run_bounces_device(p, paths, paths, 0);
+            run_bounces_device(p, paths, paths, 0, 0);
         } else if (int rc1 = run_bounces(p, paths, 0)) {
             return rc1;
         }
@@ -785,7 +793,7 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
                                                                   deferred_count, stream_pos);
                 launches++;
                 if (device_driven) {  // at most one deferred sample per pixel and wave
-                    run_bounces_device(p_wave, 0u, cp, yar_gpu_ctx::kBounceBuckets - 1);
+                    run_bounces_device(p_wave, 0u, cp, yar_gpu_ctx::kBounceBuckets - 1, tail_vertices_behind(p));
                     continue;
                 }
                 uint32_t n = 0;
@@ -1043,7 +1051,7 @@ int render_run_static(yar_gpu_ctx* ctx, float* rgb_out_device, yar_render_stats*
             e = trace_light_queues(ctx, q, ps, count, bounce, st);
             if (e != cudaSuccess) break;
             connect_kernel<<<grid_for(count), kBlock, 0, st>>>(pp, S, q.ext_slot[cur], count, ps, nullptr);
-            launches += 5;
+            launches += 5 + (ctx->ds.wide_nodes ? 3 : 0);
             uint32_t h[4];
             e = cudaMemcpyAsync(h, q.counters, sizeof(h), cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);

@@ -548,7 +548,7 @@ inline int bounce_bucket(int bounce) { return bounce < yar_gpu_ctx::kBounceBucke
 inline int render_choice(const yar_gpu_ctx* ctx, int kind, int bounce) {
     for (int b = bounce_bucket(bounce); b >= 0; b--)
         if (ctx->render_kernel[kind][b] >= 0) return ctx->render_kernel[kind][b];
-    return kCastPersistent64;
+    return ctx->ds.wide_nodes ? kCastWide : kCastPersistent64;
 }
 
 cudaError_t trace_extend(yar_gpu_ctx* ctx, const Queues& q, int cur, uint32_t count, int bounce, cudaStream_t st) {
@@ -559,6 +559,7 @@ cudaError_t trace_extend(yar_gpu_ctx* ctx, const Queues& q, int cur, uint32_t co
     a.err = reinterpret_cast<int*>(q.counters + 3);
     a.hit4 = q.ext_hit4;
     a.hit2 = q.ext_hit2;
+    a.answers = q.shd_slot;  // the shade kernel fills it later
     const int b = bounce_bucket(bounce);
     if (ctx->render_kernel[0][b] < 0 && count >= kRenderTuneMinRays) return tune_render_bucket(ctx, a, 0, b, st);
     return launch_extend(ctx->ds, a, render_choice(ctx, 0, bounce), st);
@@ -574,6 +575,7 @@ cudaError_t trace_light_queues(yar_gpu_ctx* ctx, const Queues& q, const Path_Sta
     sh.next_ray = q.counters + 5;
     sh.err = reinterpret_cast<int*>(q.counters + 3);
     sh.occluded = ps.occluded;
+    sh.answers = reinterpret_cast<uint32_t*>(q.ext_hit2);  // the shade kernel has read it
     const int b = bounce_bucket(bounce);
     cudaError_t e = (ctx->render_kernel[1][b] < 0 && count >= kRenderTuneMinRays)
                         ? tune_render_bucket(ctx, sh, 1, b, st)
@@ -588,6 +590,7 @@ cudaError_t trace_light_queues(yar_gpu_ctx* ctx, const Queues& q, const Path_Sta
     pr.err = reinterpret_cast<int*>(q.counters + 3);
     pr.hit4 = ps.probe_hit4;
     pr.hit2 = ps.probe_hit2;
+    pr.answers = reinterpret_cast<uint32_t*>(q.ext_hit2);
     return launch_extend(ctx->ds, pr, render_choice(ctx, 0, bounce), st);
 }
 
@@ -699,6 +702,15 @@ __device__ __forceinline__ bool tail_may_draw_past_budget(const Render_Params& p
     const int n1 = 3 + ((info & kDeltaArrival) && bounce >= p.rr_bounce_threshold ? 1 : 0) +
                    (bounce + 1 >= p.rr_bounce_threshold ? 1 : 0);
     return i1d + n1 > p.n1d || i2d + 3 > p.n2d;
+}
+
+// Vertices that every path has behind it when it is deferred: a vertex takes at
+// most five 1D dimensions (the two roulettes among them) and three 2D ones.  A
+// tail wave's paths are done that many bounces before a camera path's.
+inline int tail_vertices_behind(const Render_Params& p) {
+    int k = 0;
+    while (5 * k + 5 <= p.n1d && 3 * k + 3 <= p.n2d) k++;
+    return k;
 }
 
 // ---------------------------------------------------------------- triangle-mesh lights
@@ -2112,6 +2124,7 @@ __global__ void bounce_begin_kernel(uint32_t* counters, uint32_t first_paths, un
     rays[1] += prev_shadow;
     counters[7] = first_paths ? first_paths : counters[0];
     counters[0] = counters[1] = counters[2] = 0;
+    counters[4] = counters[5] = counters[6] = 0;  // the casts' hand-out counters (Cast_Args::next_ray_zeroed)
 }
 
 __global__ void __launch_bounds__(kBlock)
