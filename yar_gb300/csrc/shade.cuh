@@ -5,9 +5,8 @@
 //
 // Every expression keeps the reference's operand order; the translation unit
 // is compiled with -fmad=false and IEEE division/sqrt, so all of it rounds
-// like the reference except sin/cos: those are evaluated in double precision
-// and rounded once to float, which gives the correctly rounded float result
-// (what glibc's sinf/cosf return for all but a vanishing fraction of inputs).
+// like the reference except sin/cos: those are correctly rounded (what glibc's
+// sinf/cosf return for all but a vanishing fraction of inputs).
 #pragma once
 
 #include <cstdint>
@@ -49,8 +48,73 @@ __device__ __forceinline__ float min_std(float a, float b) { return (b < a) ? b 
 __device__ __forceinline__ float max_component(Col c) { return max_std(c.r, max_std(c.g, c.b)); }
 __device__ __forceinline__ float clamp1(float x) { return x < -1.f ? -1.f : (x > 1.f ? 1.f : x); }
 
-__device__ __forceinline__ float sin_f(float x) { return (float)sin((double)x); }
-__device__ __forceinline__ float cos_f(float x) { return (float)cos((double)x); }
+// Sines and cosines of sampled angles, correctly rounded.  In FP64 (1/64 of the
+// FP32 rate here) a vertex's took about 80 instructions that held the FP64 pipe
+// for 53% of the shade kernel's time on the Cornell box, so they
+// are evaluated as unevaluated sums of two floats: the angle reduced by
+// multiples of pi/2 (three-part constant, Cody and Waite), Taylor polynomials
+// whose first four steps are two-float products (Dekker; the products' errors by
+// FMA), about 2^-44 relative.  Where the float nearest to the sum is not the
+// same 2^-38 to either side (one argument in 8,000), or outside [-7, 7], the
+// FP64 functions decide, so the results are theirs: compared over every float
+// in [-7, 7].
+struct Two_Float {
+    float h, l;
+};
+__device__ __forceinline__ Two_Float fast_two_sum(float a, float b) {  // |a| >= |b|
+    const float h = a + b;
+    return Two_Float{h, b - (h - a)};
+}
+// c + z v, |c| larger than the product
+__device__ __forceinline__ Two_Float horner_step(float ch, float cl, Two_Float z, Two_Float v) {
+    const float q = z.h * v.h;
+    const float e = __fmaf_rn(z.h, v.l, __fmaf_rn(z.l, v.h, __fmaf_rn(z.h, v.h, -q)));
+    Two_Float r = fast_two_sum(ch, q);
+    r.l += cl + e;
+    return r;
+}
+static __device__ __noinline__ float2 sincos_fp64(float x) { return make_float2((float)sin((double)x), (float)cos((double)x)); }
+
+// (sin x, cos x)
+__device__ __forceinline__ float2 sincos_f(float x) {
+    const float k = rintf(x * 0.636619747f);
+    const float t = __fmaf_rn(-k, 1.5703125f, x);  // exact
+    const float p = k * 4.83826792e-4f;
+    const float e = __fmaf_rn(k, 4.83826792e-4f, -p);
+    // t - p, then the rest of k pi/2
+    const float s0 = t - p, b0 = s0 - t;
+    const float low = ((t - (s0 - b0)) + (-p - b0)) - __fmaf_rn(k, 2.56334407e-12f, e);
+    const Two_Float r = fast_two_sum(s0, low);
+    Two_Float z;
+    z.h = r.h * r.h;
+    z.l = __fmaf_rn(2.f * r.h, r.l, __fmaf_rn(r.h, r.h, -z.h));
+    // sin r = r + r z S(z), cos r = 1 + z C(z)
+    float u = __fmaf_rn(z.h, 1.60590444e-10f, -2.50521079e-8f);
+    Two_Float v = fast_two_sum(2.75573188e-6f, z.h * u);
+    v.l += 3.79357122e-14f;
+    v = horner_step(-1.98412701e-4f, 2.72559687e-12f, z, v);
+    v = horner_step(8.33333377e-3f, -4.34617203e-10f, z, v);
+    v = horner_step(-0.166666672f, 4.96705388e-9f, z, v);
+    Two_Float m;
+    m.h = z.h * v.h;
+    m.l = __fmaf_rn(z.h, v.l, __fmaf_rn(z.l, v.h, __fmaf_rn(z.h, v.h, -m.h)));
+    const Two_Float sn = horner_step(r.h, r.l, r, m);
+    u = __fmaf_rn(z.h, __fmaf_rn(z.h, -1.14707454e-11f, 2.08767559e-9f), -2.755732e-7f);
+    v = fast_two_sum(2.48015876e-5f, z.h * u);
+    v.l += -3.40699609e-13f;
+    v = horner_step(-1.38888892e-3f, 3.36310944e-11f, z, v);
+    v = horner_step(4.16666679e-2f, -1.24176347e-9f, z, v);
+    v = horner_step(-0.5f, 0.f, z, v);
+    const Two_Float cs = horner_step(1.f, 0.f, z, v);
+    // the floats nearest to the sums 2^-38 to either side
+    const float es = __fmaf_rn(fabsf(sn.h), 3.63797881e-12f, 6.93889390e-18f), ec = cs.h * 3.63797881e-12f;
+    const float sv = sn.h + (sn.l + es), cv = cs.h + (cs.l + ec);
+    if (!(fabsf(x) <= 7.f) || sv != sn.h + (sn.l - es) || cv != cs.h + (cs.l - ec)) return sincos_fp64(x);
+    const int q = (int)k;
+    const float a = (q & 1) ? cv : sv, b = (q & 1) ? sv : cv;
+    return make_float2((q & 2) ? -a : a, ((q + 1) & 2) ? -b : b);
+}
+__device__ __forceinline__ float cos_f(float x) { return (float)cos((double)x); }  // (arguments of any size)
 
 constexpr float kPi = 3.14159265f;  // src/lib/math.h:7
 
@@ -270,7 +334,8 @@ __device__ __forceinline__ V3 sample_hemisphere_cosine(float u0, float u1) {
     const float z = sqrtf(1.f - u0);
     const float r = sqrtf(u0);
     const float phi = 2.f * kPi * u1;
-    return v3(r * cos_f(phi), r * sin_f(phi), z);
+    const float2 sc = sincos_f(phi);
+    return v3(r * sc.y, r * sc.x, z);
 }
 
 __device__ __forceinline__ float dielectric_fresnel(float cos_i, float eta) {
@@ -463,8 +528,9 @@ __device__ __forceinline__ V3 ggx_sample_vndf(float u0, float u1, V3 wo, float a
     const V3 T2 = cross(N, T1);
     const float r = sqrtf(u0);
     const float phi = 2.f * kPi * u1;
-    const float t1 = r * cos_f(phi);
-    float t2 = r * sin_f(phi);
+    const float2 sincos_phi = sincos_f(phi);
+    const float t1 = r * sincos_phi.y;
+    float t2 = r * sincos_phi.x;
     const float s = 0.5f * (1.f + N.z);
     t2 = (1.f - s) * sqrtf(1.f - t1 * t1) + s * t2;
     const V3 nh = (mul(T1, t1) + mul(T2, t2)) + mul(N, sqrtf(max_std(0.f, 1.f - t1 * t1 - t2 * t2)));

@@ -835,10 +835,11 @@ __device__ __forceinline__ Col env_light_sample(const Scene_Dev& S, float u0, fl
     const float ky = cdf_sample(S.env_marginal, S.env_ny, u0, pdf_y, y);
     const float kx = cdf_sample(S.env_cdfs + (size_t)y * S.env_nx, S.env_nx, u1, pdf_x, x);
     const float phi = kx * 6.2831853f, theta = ky * kPi;
-    const float sin_theta = sin_f(theta);
+    const float2 sc_theta = sincos_f(theta), sc_phi = sincos_f(phi);
+    const float sin_theta = sc_theta.x;
     pdf = (pdf_y * pdf_x) / (2 * kPi * kPi * sin_theta);
     wi = xform_vector(S.env_l2w[0], S.env_l2w[1], S.env_l2w[2],
-                      v3(sin_theta * cos_f(phi), sin_theta * sin_f(phi), cos_f(theta)));
+                      v3(sin_theta * sc_phi.y, sin_theta * sc_phi.x, sc_theta.y));
     return env_nearest(S, kx, ky) * col(S.env_scale.x, S.env_scale.y, S.env_scale.z);
 }
 
@@ -1314,7 +1315,8 @@ __device__ __forceinline__ V3 sphere_sampler_sample(const Sphere_Sampler& ss, fl
     const float d_sample = ss.d_center * cos_theta - sqrtf(max_std(0.f, radius2 - d_center2 * sin_theta2));
     const float cos_alpha = (d_center2 + radius2 - d_sample * d_sample) / (2.f * ss.d_center * ss.radius);
     const float sin_alpha = sqrtf(max_std(0.f, 1.f - cos_alpha * cos_alpha));
-    const V3 dir = (mul(ss.axes[0], sin_alpha * cos_f(phi)) + mul(ss.axes[1], sin_alpha * sin_f(phi))) +
+    const float2 sc_phi = sincos_f(phi);
+    const V3 dir = (mul(ss.axes[0], sin_alpha * sc_phi.y) + mul(ss.axes[1], sin_alpha * sc_phi.x)) +
                    mul(ss.axes[2], cos_alpha);
     return mul(dir, ss.radius) + ss.center;
 }
