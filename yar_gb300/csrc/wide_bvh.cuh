@@ -292,7 +292,8 @@ struct Wide_Traversal {
             return true;
         }
         if (th < t) {
-            if (best != kWideNone && t <= th * kWideNear) flags |= 1u << 16;
+            // (every triangle accepted so far is at t or beyond)
+            flags = (flags & ~(1u << 16)) | (best != kWideNone && t <= th * kWideNear ? 1u << 16 : 0u);
             best = triangle;
             t = th;
             limit = th * kWideNear;
