@@ -183,8 +183,9 @@ cudaError_t enqueue_scene(Batch& bt, int si, bool one_spp, unsigned long long* s
     }
     const bool mixed = (seen & (seen - 1)) != 0;
     // the extend queues after the camera bounce sorted by direction octant and
-    // origin cell, in scenes up to 1M triangles (as render_run_params does)
-    const bool sort_rays = sub->tris.bytes / (3 * sizeof(float4)) <= (1u << 20);
+    // origin cell, where the kd-tree kernels trace them in scenes up to 1M
+    // triangles (as render_run_params does)
+    const bool sort_rays = sc.kernel[0] != kCastWide && sub->tris.bytes / (3 * sizeof(float4)) <= (1u << 20);
     Ray_Grid grid_box;
     for (int k = 0; k < 3; k++) {
         const float lo = sub->ds.scene_bounds[k], ext = sub->ds.scene_bounds[3 + k] - lo;
@@ -402,8 +403,8 @@ int render_batch(yar_gpu_ctx* ctx, const yar_flat_scene* const* scenes, uint32_t
             a.hit4 = dp<float4>(hits);
             a.hit2 = reinterpret_cast<uint2*>(dp<float4>(hits) + n);
             for (int kind = 0; kind < 2 && e == cudaSuccess; kind++) {
-                if (s.sub->cast_kernel[kind] >= 0) {  // fixed by the options, or the wide tree
-                    s.kernel[kind] = s.sub->cast_kernel[kind];
+                if (s.sub->render_kernel[kind][0] >= 0) {  // fixed by the options or by the scene
+                    s.kernel[kind] = s.sub->render_kernel[kind][0];
                     continue;
                 }
                 Cast_Args k = a;

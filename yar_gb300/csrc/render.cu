@@ -628,10 +628,13 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
     };
     // The rays of bounces after the camera's, sorted by direction octant and
     // origin cell into the other extend buffer (the traversal then reads
-    // that one), in scenes of at most kSortRaysMaxTriangles triangles: on C1
-    // (36 triangles) the render went from 5.50 to 5.32 ms; on C3 (4.1M
-    // triangles, a kd-tree larger than L2) the sort cost more than it saved
-    // (1.323-1.345 s against 1.311 s).
+    // that one), where the kd-tree kernels trace them and the scene has at
+    // most kSortRaysMaxTriangles triangles: the GGX room takes 42.4 ms sorted,
+    // 44.4 ms unsorted; on a kd-tree larger than L2 the sort cost more than it
+    // saved (4.1M triangles: 1.323-1.345 s against 1.311 s).  The wide tree's
+    // kernel refills its lanes one by one and gains nothing from the order
+    // (Cornell box 2.84 ms unsorted, 3.14 ms sorted; 4.1M triangles 84.5 ms,
+    // 89.1 ms).
     Ray_Grid grid_box;
     for (int k = 0; k < 3; k++) {
         const float lo = ctx->ds.scene_bounds[k], ext = ctx->ds.scene_bounds[3 + k] - lo;
@@ -639,7 +642,7 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
         grid_box.scale[k] = ext > 0.f ? 8.f / ext : 0.f;
     }
     constexpr uint64_t kSortRaysMaxTriangles = 1u << 20;
-    const bool sort_rays = ctx->tris.bytes / (3 * sizeof(float4)) <= kSortRaysMaxTriangles;
+    const bool sort_rays = render_choice(ctx, 0, 1) != kCastWide && ctx->tris.bytes / (3 * sizeof(float4)) <= kSortRaysMaxTriangles;
     uint16_t* ray_keys = dptr<uint16_t>(B[40]);
     uint32_t* ray_hist = dptr<uint32_t>(B[41]);
     auto sort_queue = [&](int from, const uint32_t* count_dev, uint32_t count, uint32_t max_count) {
