@@ -319,8 +319,8 @@ extern "C" int yar_gpu_upload_scene(yar_gpu_ctx* ctx, const yar_flat_scene* scen
     // any hit 3.2 against 11.2), but renders of a scene of tessellated planes
     // walk the kd-tree, one ray per thread: the render's rays reach a plane
     // together, and there a binary descent takes fewer instructions than eight
-    // boxes a level (the GGX room at 512 x 512, 64 samples: 44.9 ms against
-    // 50.3 ms; already with 800 triangles a wall any-hit rays are faster).
+    // boxes a level (the GGX room at 512 x 512, 64 samples: 42.4 ms against
+    // 43.1 ms; equal at 3,200 triangles a wall).
     int fixed = ctx->forced_kernel;
     if (fixed < 0) {
         e = wide_build(ctx, scene, tri_offset.data(), node_offset.data());

@@ -38,7 +38,7 @@ constexpr int kSmall = 1024;  // clusters one block finishes
 constexpr int kMaxRounds = 256;
 constexpr uint32_t kInnerBit = 0x80000000u;
 
-constexpr uint32_t kPlanarTriangles = 1024;  // of a scene of tessellated planes (yar_gpu_ctx::wide_planar)
+constexpr uint32_t kPlanarTriangles = 16384;  // of a scene of tessellated planes (yar_gpu_ctx::wide_planar)
 
 struct Build_Object {
     uint32_t first;       // of its primitives
