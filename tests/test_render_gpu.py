@@ -283,6 +283,28 @@ def test_render_direct_lighting_sphere_lights_bit_identical(gpu_ctx, samples):
     assert stats.variance == ref_var
 
 
+@pytest.mark.parametrize("scene,width,height,rect_samples",
+                         [("cornell_direct_64", 64, 64, 289), ("cornell_direct_64", 521, 509, 4),
+                          ("cornell_direct_env_64", 521, 509, 1)])
+def test_render_direct_lighting_split_over_launches(gpu_ctx, scene, width, height, rect_samples):
+    """The light samples of a chunk split over several launches (inside a
+    light's sample array), and an image of more than one chunk: as the oracle."""
+    s = FlatScene.read(golden(scene + ".yfs"))
+    s.camera = np.array(s.camera)
+    s.config = np.array(s.config)
+    s.camera["image_extent"] = (width, height)
+    s.camera["horz_half_dist"] = np.float32(np.float32(width) / np.float32(height)) * s.camera["vert_half_dist"]
+    s.config["render_region"] = (0, 0, width, height)
+    rl = s.rect_lights.copy()
+    rl["sample_count"] = rect_samples
+    s.rect_lights = rl
+    ref, ref_var = oracle.render(s, threads=8, correctly_rounded_trig=True)
+    gpu_ctx.upload_scene(s)
+    img, stats = gpu_ctx.render(width, height)
+    assert np.array_equal(img.view(np.uint32), ref.view(np.uint32))
+    assert stats.variance == ref_var
+
+
 def test_render_unsupported_features_fail_cleanly(gpu_ctx):
     from yar_gb300 import native
     s = FlatScene.read(golden("cornell_c1_64.yfs"))
