@@ -209,3 +209,46 @@ def test_bounded_wait_gives_up_and_the_context_stays_usable(gpu_ctx):
     gpu_ctx.guide_infer(q.data_ptr(), n, BOX, lobes.data_ptr())
     got = lobes.cpu().numpy().reshape(n, 8, 5)
     assert np.allclose(got[:, :, 4].sum(1), 1.0, atol=1e-5)
+
+
+@pytest.mark.parametrize("n", [31, 33, 152 * 128 + 1, 2 * 152 * 128, 5 * 152 * 128 + 97, 6 * 152 * 128 + 1])
+def test_inference_over_the_groups_of_a_cta(gpu_ctx, n):
+    """Rows that fill the first group of every CTA, all five, and more than one
+    tile per group; nothing behind the last row is written."""
+    params = random_params(11)
+    gpu_ctx.guide_set_params(params)
+    rows = random_rows(n, 12)
+    q = device(rows)
+    lobes = torch.full((n + 32, 40), -7.0, dtype=torch.float32, device="cuda")
+    gpu_ctx.guide_infer(q.data_ptr(), n, BOX, lobes.data_ptr())
+    assert torch.all(lobes[n:] == -7.0)
+    got = lobes[:n].cpu().numpy().reshape(n, 8, 5)
+    with torch.no_grad():
+        o, _ = forward(params, rows)
+        mu, kappa, logpi = mixture(o)
+        mlen = o[:, 0:40].reshape(-1, 8, 5)[:, :, 0:3].norm(dim=2)
+    assert (np.abs(got[:, :, 0:3] - mu.numpy()).max(2) * mlen.numpy()).max() < LOBE_ABS_TOL
+    assert np.abs(np.log(got[:, :, 3]) - kappa.log().numpy()).max() < LOBE_ABS_TOL
+    assert np.abs(got[:, :, 4] - torch.exp(logpi).numpy()).max() < LOBE_ABS_TOL
+
+
+@pytest.mark.parametrize("n", [1, 129, 152 * 128 + 1, 2 * 152 * 128, 2 * 152 * 128 + 130, 3 * 152 * 128 - 5])
+def test_gradient_over_the_groups_of_a_cta(gpu_ctx, n):
+    """Rows for one, two and three tiles per CTA: each of its two groups with
+    and without a tile of its own."""
+    params = random_params(13)
+    gpu_ctx.guide_set_params(params)
+    rows = random_rows(n, 14, train=True)
+    s = device(rows)
+    grad = torch.full((native.GUIDE_PARAMS,), -7.0, dtype=torch.float32, device="cuda")
+    loss = gpu_ctx.guide_gradient(s.data_ptr(), n, BOX, 1.0 / n, grad.data_ptr())
+    got = grad.cpu().numpy()
+    o, ws = forward(params, rows, grad=True)
+    ref = -(torch.as_tensor(rows[:, 12]) / n * log_q(o, rows[:, 9:12])).sum()
+    ref.backward()
+    assert abs(loss - ref.item()) <= LOSS_REL_TOL * abs(ref.item()) + 1e-3
+    want = [w.grad.ravel().numpy() for w in ws]
+    for i, (w, at) in enumerate(zip(want, (0, 8192, 12288, 16384))):
+        g = got[at:at + len(w)]
+        assert np.linalg.norm(g - w) < GRAD_REL_TOL * np.linalg.norm(w), (i, n)
+    assert np.all(got[16384 + 40 * 64:] == 0.0)

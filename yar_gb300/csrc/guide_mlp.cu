@@ -11,14 +11,15 @@
 // per lobe an unnormalised mean direction m (3), log-concentration r and a
 // mixture logit l.  kappa = exp(clamp(r, -3, 8)), pi = softmax(l).
 //
-// One CTA of 128 threads handles tiles of 128 rows (= TMEM lanes = threads);
-// a single thread issues the MMAs (M = 128, N = 64, K = 16 per instruction),
-// all threads run the epilogues (tcgen05.ld of their lane, bias-free ReLU,
-// BF16 pack into the next layer's operand tile).  Training fuses the forward
-// pass, the loss gradient, the backward pass and the weight gradients: the
-// weight gradients dW^T = A^T dY accumulate in tensor memory over all tiles a
-// CTA processes (the transposed operand tiles are written by the epilogues),
-// and each CTA writes one partial gradient; adam_kernel sums the partials.
+// A group of 128 threads handles a tile of 128 rows (= TMEM lanes = threads):
+// one thread issues the MMAs (M = 128, N = 64, K = 16 per instruction), all
+// threads run the epilogues (tcgen05.ld of their lane, bias-free ReLU, BF16
+// pack into the next layer's operand tile).  Several groups share a CTA and
+// its copy of the weights, so that one group's epilogue runs while another's
+// MMA is in flight.  Training fuses the forward pass, the loss gradient, the
+// backward pass and the weight gradients: the weight gradients dW^T = A^T dY
+// accumulate in tensor memory over all tiles a CTA processes, and each CTA
+// writes one partial gradient; adam_kernel sums the partials.
 //
 // Loss for a sample direction w drawn with pdf p at (x, n, wo) with target
 // value t (incident radiance x BSDF x cosine, as luminance): -(t / p) log q(w),
@@ -50,27 +51,33 @@ constexpr int kW3 = kW2 + kHid * kHid;
 constexpr int kW4 = kW3 + kHid * kHid;
 static_assert(kW4 + kOut * kHid == kGuideParams, "parameter count");
 
-// bf16 operand images in tile layout: W1 (64 x 128), W2..W4 (64 x 64), then
-// the transposed W2..W4 (rows = input unit, K = output unit) for the backward pass
-constexpr uint32_t kImgW1 = 0, kImgW2 = 16384, kImgW3 = 24576, kImgW4 = 32768;
-constexpr uint32_t kImgW2t = 40960, kImgW3t = 49152, kImgW4t = 57344, kImgBytes = 65536;
+// bf16 operand images in tile layout: W1 (64 x 128), W2..W4 (64 x 64), rows =
+// output unit.  Every tile serves as a K-major operand (rows x columns) and,
+// with the MN-major bit, as its transpose: its 8 x 8 core matrices are the
+// same in both, only the roles of the two strides change.  So the backward
+// pass reads W as W^T, and the weight gradients read the activation and
+// gradient rows as A^T and dY, without transposed copies.
+constexpr uint32_t kImgW1 = 0, kImgW2 = 16384, kImgW3 = 24576, kImgW4 = 32768, kImgBytes = 40960;
+constexpr int kGradOut = 48;  // columns of the output gradient's tile: the 40 outputs, then zeros
 
-// shared memory, training: images | R0 (32 KB rows) | H1t H2t H3t dT (16 KB each) | Xt (32 KB) | misc
-// H_t tiles hold 64 rows but the M = 128 MMA reads 128: rows 64..127 come
-// from the next tile in this list (their products land in TMEM lanes that
-// are never read).
-constexpr uint32_t kTrR0 = kImgBytes;
-constexpr uint32_t kTrH1t = kTrR0 + 32768;
-constexpr uint32_t kTrH2t = kTrH1t + 16384;
-constexpr uint32_t kTrH3t = kTrH2t + 16384;
-constexpr uint32_t kTrDT = kTrH3t + 16384;
-constexpr uint32_t kTrXt = kTrDT + 16384;
-constexpr uint32_t kTrMisc = kTrXt + 32768;
-// shared memory, inference: W1..W4 images | R0 | misc
-constexpr uint32_t kInR0 = kImgW2t;
-constexpr uint32_t kInMisc = kInR0 + 32768;
+// shared memory, training: images | per group: X (32 KB), H1 H2 H3 (16 KB
+// each; each is overwritten by its gradient), dOut (12 KB) | misc.  H tiles
+// hold 64 columns but the transposed M = 128 operand reads 128: columns 64 to
+// 127 come from the following rows, at the end of a tile from the tile behind
+// it (their products land in TMEM lanes that are never read).
+constexpr int kTrGroups = 2;
+constexpr uint32_t kTrX = 0, kTrH = 32768, kTrDOut = kTrH + 3 * 16384, kTrGroupBytes = kTrDOut + kRows * kGradOut * 2;
+constexpr uint32_t kTrMisc = kImgBytes + kTrGroups * kTrGroupBytes;
+constexpr int kTrThreads = kTrGroups * kRows + 32;  // and a warp that issues the MMAs
+// shared memory, inference: images | per group 32 KB of rows | misc
+constexpr int kInGroups = 5;
+constexpr uint32_t kInMisc = kImgBytes + kInGroups * 32768u;
+constexpr int kInThreads = kInGroups * kRows;
+constexpr uint32_t kMiscBytes = 192;  // 0: barriers, 96: TMEM address, 100: abort flag, 128: drain barriers
+static_assert(kTrMisc + kMiscBytes <= 232448 && kInMisc + kMiscBytes <= 232448, "227 KB of shared memory");
 
-constexpr uint32_t kIdesc = tc::idesc_bf16_f32(128, 64);
+// kind::f16 instruction descriptors: operands K-major, or read as their transpose
+constexpr uint32_t kTransA = 1u << 15, kTransB = 1u << 16;
 
 struct Mlp_Args {
     const uint8_t* images;
@@ -105,8 +112,8 @@ __constant__ float kFreq[3] = {1.000000000e+00f, 1.259921074e+00f, 1.587401032e+
 struct Encoding {
     float s[3][3], c[3][3];  // running sin and cos per (axis, chain)
 };
-__device__ __forceinline__ void feature_pair(int j, float3 p, float3 nrm, float3 wo, bool valid, Encoding& e,
-                                             float& f0, float& f1) {
+__device__ __forceinline__ void feature_pair(int j, float3 p, float3 nrm, float3 wo, Encoding& e, float& f0,
+                                             float& f1) {
     if (j < 96) {
         const int k = j / 6, a = (j % 6) / 2, b = k % 3;
         if (k < 3) {
@@ -117,12 +124,8 @@ __device__ __forceinline__ void feature_pair(int j, float3 p, float3 nrm, float3
             e.s[a][b] = 2.f * sn * cs;
             e.c[a][b] = (cs - sn) * (cs + sn);
         }
-        f0 = valid ? e.s[a][b] : 0.f;
-        f1 = valid ? e.c[a][b] : 0.f;
-        return;
-    }
-    if (!valid) {
-        f0 = f1 = 0.f;
+        f0 = e.s[a][b];
+        f1 = e.c[a][b];
         return;
     }
     auto fixed = [&](int i) -> float {
@@ -141,13 +144,6 @@ __device__ __forceinline__ void feature_pair(int j, float3 p, float3 nrm, float3
     f1 = fixed(j + 1);
 }
 
-// Transposed tile write: element (feature f, batch row r) of a tile with
-// K = 128 batch columns; neighbouring rows pair up into one 4-byte store.
-__device__ __forceinline__ void store_t(uint8_t* tile, int f, int r, float v) {
-    const float u = __shfl_down_sync(0xffffffffu, v, 1);
-    if ((r & 1) == 0) *reinterpret_cast<uint32_t*>(tile + tc::tile_offset(f, r, 128)) = pack_bf16(v, u);
-}
-
 __device__ __forceinline__ void store_row8(uint8_t* tile, int r, int k0, int K, const float* v) {
     uint4 q;
     q.x = pack_bf16(v[0], v[1]);
@@ -157,37 +153,134 @@ __device__ __forceinline__ void store_row8(uint8_t* tile, int r, int k0, int K, 
     *reinterpret_cast<uint4*>(tile + tc::tile_offset(r, k0, K)) = q;
 }
 
-// A tile (M = 128 rows, K = ksteps * 16) times a B tile (N = 64 rows, same K).
-__device__ __forceinline__ void gemm(uint32_t d_tmem, uint32_t a, uint32_t b, int K, bool accumulate) {
-    const uint32_t sbo = (uint32_t)K * 16u;
-    for (int s = 0; s < K / 16; s++) {
-        const uint64_t ad = tc::smem_desc(a + 256u * s, 128u, sbo);
-        const uint64_t bd = tc::smem_desc(b + 256u * s, 128u, sbo);
-        tc::mma(d_tmem, ad, bd, kIdesc, (accumulate || s > 0) ? 1u : 0u);
-    }
+// An MMA operand over K = 16 * n: a tile of `cols` columns, its rows the M or
+// N dimension (K-major), or its columns (MN-major, `trans`).
+struct Operand {
+    uint32_t addr, cols;
+    bool trans;
+};
+__device__ __forceinline__ uint64_t operand_desc(const Operand& o, int k16) {
+    const uint32_t rows8 = o.cols * 16u;  // from 8 rows to the next 8
+    return o.trans ? tc::smem_desc(o.addr + 2u * rows8 * (uint32_t)k16, rows8, 128u)
+                   : tc::smem_desc(o.addr + 256u * (uint32_t)k16, 128u, rows8);
+}
+__device__ __forceinline__ void gemm(uint32_t d_tmem, Operand a, Operand b, int K, int N, bool accumulate) {
+    const uint32_t idesc = tc::idesc_bf16_f32(128, N) | (a.trans ? kTransA : 0u) | (b.trans ? kTransB : 0u);
+    for (int s = 0; s < K / 16; s++)
+        tc::mma(d_tmem, operand_desc(a, s), operand_desc(b, s), idesc, (accumulate || s > 0) ? 1u : 0u);
 }
 
-__device__ __forceinline__ void load64(uint32_t taddr, float (&v)[64]) {
-    float* p = v;
-    tc::tmem_ld16(taddr + 0, *reinterpret_cast<float(*)[16]>(p + 0));
-    tc::tmem_ld16(taddr + 16, *reinterpret_cast<float(*)[16]>(p + 16));
-    tc::tmem_ld16(taddr + 32, *reinterpret_cast<float(*)[16]>(p + 32));
-    tc::tmem_ld16(taddr + 48, *reinterpret_cast<float(*)[16]>(p + 48));
+template <int N>
+__device__ __forceinline__ void load_row(uint32_t taddr, float (&v)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; i += 16) tc::tmem_ld16(taddr + i, *reinterpret_cast<float(*)[16]>(v + i));
     tc::tmem_wait_ld();
 }
 
-// Issue barrier: the generic-proxy shared-memory writes of all threads become
-// visible to the tensor core, and tensor-memory reads of the epilogue are
-// ordered before the next MMA.
-__device__ __forceinline__ void to_mma() {
+// Before an MMA: the generic-proxy shared-memory writes of this thread become
+// visible to the tensor core, and its tensor-memory reads are ordered before
+// the MMA; `ready` counts the group's threads.
+__device__ __forceinline__ void arrive_ready(uint32_t ready) {
     tc::fence_proxy_async();
     tc::fence_before_sync();
-    __syncthreads();
+    tc::mbar_arrive(ready);
+}
+
+// Bounded wait; gives up at once when another thread has given up.
+__device__ __forceinline__ bool wait_or_abort(uint32_t mbar, uint32_t parity, volatile int* abort) {
+    for (uint32_t i = 0; i < kWaitLimit / 64u; i++) {
+        if (tc::mbar_wait(mbar, parity, 64u)) return true;
+        if (*abort) return false;
+    }
+    *abort = 1;
+    return false;
+}
+
+// After giving up: the MMAs that this thread has issued finish (or the wait's
+// limit runs out) before the tensor memory is freed.
+__device__ __forceinline__ void drain(uint32_t mbar) {
+    tc::commit(mbar);
+    tc::mbar_wait(mbar, 0u, kWaitLimit);
+}
+
+// A row of the input (3 float4 a query, 4 a training sample).
+struct Input {
+    float3 p, nrm, wo, wdir;
+    float wt;
+};
+template <bool TRAIN>
+__device__ __forceinline__ Input load_input(const Mlp_Args& a, uint32_t row, bool valid, float w_scale) {
+    Input x;
+    x.p = x.nrm = x.wo = x.wdir = make_float3(0.f, 0.f, 0.f);
+    x.wt = 0.f;
+    if (valid) {
+        const float4* q = a.rows + ((size_t)a.offset + (size_t)row * a.stride) * (TRAIN ? 4 : 3);
+        const float4 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2);
+        x.p = make_float3((q0.x - a.lo.x) * a.inv_ext.x, (q0.y - a.lo.y) * a.inv_ext.y,
+                          (q0.z - a.lo.z) * a.inv_ext.z);
+        x.nrm = make_float3(q0.w, q1.x, q1.y);
+        x.wo = make_float3(q1.z, q1.w, q2.x);
+        if (TRAIN) {
+            x.wdir = make_float3(q2.y, q2.z, q2.w);
+            x.wt = __ldg(q + 3).x * w_scale;
+        }
+    }
+    return x;
+}
+
+// The input features of this thread's row into the tile X.
+__device__ __forceinline__ void store_features(uint8_t* X, int r, const Input& x) {
+    Encoding enc;
+#pragma unroll
+    for (int c = 0; c < 16; c++) {
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) feature_pair(8 * c + i, x.p, x.nrm, x.wo, enc, v[i], v[i + 1]);
+        store_row8(X, r, 8 * c, kIn, v);
+    }
+}
+
+// ReLU of a row of 64 sums into the operand tile H; unit 63 is the constant 1.
+// The maximum is taken on the rounded pairs (rounding keeps the order).
+__device__ __forceinline__ void store_hidden(uint8_t* H, int r, const float (&v)[64]) {
+    const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+        uint32_t q[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int j = 8 * c + 2 * i;
+            const __nv_bfloat162 h = __hmax2(__floats2bfloat162_rn(v[j], j == 62 ? 1.f : v[j + 1]), zero);
+            q[i] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        *reinterpret_cast<uint4*>(H + tc::tile_offset(r, 8 * c, kHid)) = make_uint4(q[0], q[1], q[2], q[3]);
+    }
+}
+
+// A row of 64 gradients, zero where the unit's ReLU is (and for the constant
+// unit), over that unit's activations in the tile H.
+__device__ __forceinline__ void store_hidden_grad(uint8_t* H, int r, const float (&v)[64]) {
+    const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+        uint4* at = reinterpret_cast<uint4*>(H + tc::tile_offset(r, 8 * c, kHid));
+        const uint4 h4 = *at;
+        const uint32_t h[4] = {h4.x, h4.y, h4.z, h4.w};
+        uint32_t q[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int j = 8 * c + 2 * i;
+            const uint32_t on = __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&h[i]), zero);
+            q[i] = pack_bf16(v[j], v[j + 1]) & (j == 62 ? on & 0xffffu : on);
+        }
+        *at = make_uint4(q[0], q[1], q[2], q[3]);
+    }
 }
 
 // Mixture parameters and the loss gradient of one row (training) from the 40
 // raw outputs; `d` receives d(loss)/d(raw).
-__device__ __forceinline__ float mixture_grad(const float (&o)[64], float3 w_dir, float wt, float (&d)[64]) {
+__device__ __forceinline__ float mixture_grad(const float (&o)[kGradOut], float3 w_dir, float wt,
+                                              float (&d)[kGradOut]) {
     float lp[8], lv[8], kap[8], len[8], cdot[8], inrange[8];
     float3 mu[8];
     float lmax = -1e30f;
@@ -218,7 +311,7 @@ __device__ __forceinline__ float mixture_grad(const float (&o)[64], float3 w_dir
     for (int k = 0; k < 8; k++) qs += __expf(lp[k] + lv[k] - qmax);
     const float logq = qmax + __logf(qs);
 #pragma unroll
-    for (int j = 0; j < 64; j++) d[j] = 0.f;
+    for (int j = 40; j < kGradOut; j++) d[j] = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; k++) {
         const float gam = __expf(lp[k] + lv[k] - logq);
@@ -235,221 +328,274 @@ __device__ __forceinline__ float mixture_grad(const float (&o)[64], float3 w_dir
     return -wt * logq;
 }
 
-template <bool TRAIN>
-__global__ void __launch_bounds__(kRows, 1) mlp_kernel(Mlp_Args a) {
-    extern __shared__ __align__(1024) uint8_t sm[];
-    const int tid = threadIdx.x, warp = tid >> 5;
+// Weight images into shared memory, barriers, tensor memory; returns its address.
+template <int GROUPS>
+__device__ __forceinline__ uint32_t mlp_begin(const Mlp_Args& a, uint8_t* sm, uint32_t misc, uint32_t ready_count) {
     const uint32_t base = tc::smem_addr(sm);
-    const uint32_t misc = TRAIN ? kTrMisc : kInMisc;
-    const uint32_t mbar = base + misc;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + misc + 8);
-    constexpr uint32_t kCols = TRAIN ? 512u : 64u;
-
-    const uint32_t img_bytes = TRAIN ? kImgBytes : kImgW2t;
-    for (uint32_t i = tid; i < img_bytes / 16; i += kRows)
+    for (uint32_t i = threadIdx.x; i < kImgBytes / 16; i += blockDim.x)
         reinterpret_cast<uint4*>(sm)[i] = __ldg(reinterpret_cast<const uint4*>(a.images) + i);
-    if (warp == 0) tc::tmem_alloc(base + misc + 8, kCols);
-    if (tid == 0) {
-        tc::mbar_init(mbar, 1);
+    if (threadIdx.x < 32) tc::tmem_alloc(base + misc + 96, 512u);
+    if (threadIdx.x == 0) {
+        for (int g = 0; g < GROUPS; g++) {
+            tc::mbar_init(base + misc + 16 * g, ready_count);
+            tc::mbar_init(base + misc + 16 * g + 8, 1);
+            tc::mbar_init(base + misc + 128 + 8 * g, 1);
+        }
+        *reinterpret_cast<int*>(sm + misc + 100) = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    tc::fence_proxy_async();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t tmem = *tmem_slot;
-    const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
+    return *reinterpret_cast<uint32_t*>(sm + misc + 96);
+}
+__device__ __forceinline__ uint32_t mlp_rows(const Mlp_Args& a) {
+    return a.count ? (*a.count > a.offset ? (*a.count - a.offset + a.stride - 1) / a.stride : 0u) : a.n;
+}
 
-    const uint32_t n = a.count ? (*a.count > a.offset ? (*a.count - a.offset + a.stride - 1) / a.stride : 0u) : a.n;
-    const uint32_t tiles = (n + kRows - 1) / kRows;
-    const uint32_t r0 = base + (TRAIN ? kTrR0 : kInR0);
-    uint8_t* R0 = sm + (TRAIN ? kTrR0 : kInR0);
+// Inference.  A tile is a serial chain (features, 4 MMAs, 4 epilogues; 1,500
+// instructions per row), so the tiles in flight per SM set the rate: 5 groups
+// on one copy of the weights, where 3 CTAs of one group with their own copies
+// fitted.  The results leave through shared memory (16-byte stores 160 bytes
+// apart took 320 of the 480 shared-memory and store cycles of a warp's rows).
+// 1M rows: 137 us with 3 CTAs per SM, 120 us with 5 groups, 92 us with both;
+// 52% of the issue slots, 32 us at the copy bandwidth.
+__global__ void __launch_bounds__(kInThreads, 1) mlp_infer_kernel(Mlp_Args a) {
+    extern __shared__ __align__(1024) uint8_t sm[];
+    const uint32_t tmem = mlp_begin<kInGroups>(a, sm, kInMisc, kRows);
+    const int group = threadIdx.x / kRows, tid = threadIdx.x % kRows;
+    const uint32_t base = tc::smem_addr(sm);
+    const uint32_t ready = base + kInMisc + 16 * group, done = ready + 8;
+    volatile int* abort = reinterpret_cast<volatile int*>(sm + kInMisc + 100);
+    const uint32_t d_tmem = tmem + 64u * group;
+    const uint32_t lane_addr = d_tmem + ((uint32_t)(tid & ~31) << 16);
+    const uint32_t r_off = kImgBytes + 32768u * group;
+    uint8_t* R = sm + r_off;  // X, then the hidden layers' rows in its halves
+    // a warp's results on their way out: where its own rows of X are
+    constexpr uint32_t kLobeBytes = kGuideLobeFloats * 4u;
+    static_assert(kGuideLobeFloats == 40 && 32u * kLobeBytes <= 32u * kIn * 2u, "a warp's rows");
+    uint8_t* out = R + (tid / 32) * (32 * kIn * 2);
+    const uint32_t n = mlp_rows(a), tiles = (n + kRows - 1) / kRows;
     uint32_t parity = 0;
     bool ok = true;
-    uint32_t done_tiles = 0;
-    float loss_sum = 0.f;
-    const float w_scale = TRAIN ? __ldg(a.w_scale) : 0.f;
-
-    auto wait_mma = [&]() {
-        const bool got = tc::mbar_wait(mbar, parity, kWaitLimit);
+    // D = A * W^T of the group's tile
+    auto product = [&](uint32_t a_off, uint32_t w_off, uint32_t K) {
+        arrive_ready(ready);
+        if (tid == 0 && wait_or_abort(ready, parity, abort)) {
+            tc::fence_after_sync();
+            gemm(d_tmem, Operand{base + a_off, K, false}, Operand{base + w_off, K, false}, (int)K, kHid, false);
+            tc::commit(done);
+        }
+        const bool got = __all_sync(0xffffffffu, wait_or_abort(done, parity, abort));
         parity ^= 1u;
         tc::fence_after_sync();
         return got;
     };
-
-    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const uint32_t row = tile * kRows + tid;
+    for (uint32_t t = group; ok; t += kInGroups) {
+        const uint64_t tile = blockIdx.x + (uint64_t)t * gridDim.x;
+        if (tile >= tiles) break;
+        const uint32_t row = (uint32_t)tile * kRows + tid;
         const bool valid = row < n;
-        float3 p = make_float3(0.f, 0.f, 0.f), nrm = p, wo = p, wdir = p;
-        float wt = 0.f;
-        if (valid) {
-            const float4* q = a.rows + ((size_t)a.offset + (size_t)row * a.stride) * (TRAIN ? 4 : 3);
-            const float4 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2);
-            p = make_float3((q0.x - a.lo.x) * a.inv_ext.x, (q0.y - a.lo.y) * a.inv_ext.y,
-                            (q0.z - a.lo.z) * a.inv_ext.z);
-            nrm = make_float3(q0.w, q1.x, q1.y);
-            wo = make_float3(q1.z, q1.w, q2.x);
-            if (TRAIN) {
-                wdir = make_float3(q2.y, q2.z, q2.w);
-                wt = __ldg(q + 3).x * w_scale;
-            }
-        }
-        // ---- input features: X rows (and X^T for the weight gradient of layer 1)
-        Encoding enc;
-#pragma unroll
-        for (int c = 0; c < 16; c++) {
-            float v[8];
-#pragma unroll
-            for (int i = 0; i < 8; i += 2) feature_pair(8 * c + i, p, nrm, wo, valid, enc, v[i], v[i + 1]);
-            store_row8(R0, tid, 8 * c, kIn, v);
-            if (TRAIN) {
-#pragma unroll
-                for (int i = 0; i < 8; i++) store_t(sm + kTrXt, 8 * c + i, tid, v[i]);
-            }
-        }
-        to_mma();
-        if (tid == 0) {
-            tc::fence_after_sync();
-            gemm(tmem, r0, base + kImgW1, kIn, false);
-            tc::commit(mbar);
-        }
-        ok = wait_mma();
-        uint32_t mask[3][2];
-        // ---- hidden layers
+        const Input x = load_input<false>(a, row, valid, 0.f);
+        if ((tid & 31) == 0) tc::bulk_wait_read();  // the last tile's results have left `out`
+        __syncwarp();
+        store_features(R, tid, x);
+        ok = product(r_off, kImgW1, kIn);
+        uint32_t w_off = kImgW2;
 #pragma unroll 1
-        for (int l = 0; l < 3; l++) {
+        for (int l = 0; l < 3 && ok; l++) {
             float v[64];
-            load64(lane_addr, v);
-            mask[l][0] = mask[l][1] = 0u;
-#pragma unroll
-            for (int j = 0; j < 64; j++) {
-                if (j < 63) {
-                    if (v[j] > 0.f) mask[l][j >> 5] |= 1u << (j & 31);
-                    v[j] = fmaxf(v[j], 0.f);
-                } else {
-                    v[j] = valid ? 1.f : 0.f;
-                }
-            }
-            // layer l's output: rows into R0 (ping-pong halves), transposed into H(l+1)t
-            uint8_t* dst = R0 + ((l & 1) ? 16384 : 0);
-#pragma unroll
-            for (int c = 0; c < 8; c++) store_row8(dst, tid, 8 * c, kHid, v + 8 * c);
-            if (TRAIN) {
-                uint8_t* ht = sm + kTrH1t + 16384u * l;
-#pragma unroll
-                for (int j = 0; j < 64; j++) store_t(ht, j, tid, v[j]);
-            }
-            to_mma();
-            if (tid == 0) {
-                tc::fence_after_sync();
-                const uint32_t w = base + (l == 0 ? kImgW2 : (l == 1 ? kImgW3 : kImgW4));
-                gemm(tmem, r0 + ((l & 1) ? 16384u : 0u), w, kHid, false);
-                tc::commit(mbar);
-            }
-            ok = wait_mma() && ok;
+            load_row(lane_addr, v);
+            store_hidden(R + 16384 * (l & 1), tid, v);
+            ok = product(r_off + 16384u * (l & 1), w_off, kHid);
+            w_off += 8192u;
         }
-        // ---- output layer: mixture parameters (inference) or loss gradient (training)
-        {
-            float o[64];
-            load64(lane_addr, o);
-            if (!TRAIN) {
-                if (valid) {
-                    float lmax = -1e30f;
+        if (!ok) break;
+        float o[kGradOut];
+        load_row(lane_addr, o);
+        if (valid) {
+            float lmax = -1e30f;
 #pragma unroll
-                    for (int k = 0; k < 8; k++) lmax = fmaxf(lmax, o[5 * k + 4]);
-                    float e[8], es = 0.f;
+            for (int k = 0; k < 8; k++) lmax = fmaxf(lmax, o[5 * k + 4]);
+            float e[8], es = 0.f;
 #pragma unroll
-                    for (int k = 0; k < 8; k++) {
-                        e[k] = __expf(o[5 * k + 4] - lmax);
-                        es += e[k];
+            for (int k = 0; k < 8; k++) {
+                e[k] = __expf(o[5 * k + 4] - lmax);
+                es += e[k];
+            }
+            float f[40];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const float mx = o[5 * k], my = o[5 * k + 1], mz = o[5 * k + 2];
+                const float il = 1.f / (sqrtf(mx * mx + my * my + mz * mz) + 1e-6f);
+                f[5 * k + 0] = mx * il;
+                f[5 * k + 1] = my * il;
+                f[5 * k + 2] = mz * il;
+                f[5 * k + 3] = __expf(fminf(fmaxf(o[5 * k + 3], -3.f), 8.f));
+                f[5 * k + 4] = e[k] / es;
+            }
+#pragma unroll
+            for (int i = 0; i < 10; i++)
+                reinterpret_cast<float4*>(out + (tid & 31) * kLobeBytes)[i] =
+                    make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]);
+        }
+        tc::fence_proxy_async();
+        __syncwarp();
+        const uint32_t row0 = (uint32_t)tile * kRows + (tid & ~31);
+        if ((tid & 31) == 0 && row0 < n)
+            tc::bulk_store(a.lobes + (size_t)row0 * kGuideLobeFloats, tc::smem_addr(out),
+                           min(n - row0, 32u) * kLobeBytes);
+    }
+    if ((tid & 31) == 0) tc::bulk_wait_all();
+    __syncwarp();
+    if (!ok) {
+        atomicOr(a.err, 2);
+        if (tid == 0) drain(base + kInMisc + 128 + 8 * group);
+        __syncwarp();
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    if (threadIdx.x < 32) tc::tmem_dealloc(tmem, 512u);
+}
+
+// Training.  Two groups per CTA, each on every other tile of the CTA's, and a
+// warp that issues the MMAs of both in a fixed order: the weight gradients of
+// both accumulate in the same tensor-memory columns, tile after tile.  With
+// transposed copies of every operand (shuffles and 4-byte stores, 40% of the
+// instructions, and shared memory for one tile only) 262,144 rows took 219 us;
+// now 98 us: 3,400 instructions per row at 2 warps per scheduler, 26% of the
+// issue slots.
+__global__ void __launch_bounds__(kTrThreads, 1) mlp_train_kernel(Mlp_Args a) {
+    extern __shared__ __align__(1024) uint8_t sm[];
+    const uint32_t tmem = mlp_begin<kTrGroups>(a, sm, kTrMisc, kRows);
+    const int group = threadIdx.x / kRows, tid = threadIdx.x % kRows;
+    const uint32_t base = tc::smem_addr(sm);
+    volatile int* abort = reinterpret_cast<volatile int*>(sm + kTrMisc + 100);
+    const uint32_t n = mlp_rows(a), tiles = (n + kRows - 1) / kRows;
+    // this CTA's tiles: blockIdx.x, blockIdx.x + gridDim.x, ...
+    const uint32_t mine = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
+    const uint32_t grads = tmem + 64u * kTrGroups;  // dW1^T, then dW2^T, dW3^T, dW4^T: 64 columns each
+    bool ok = true;
+    float loss_sum = 0.f;
+    if (group == kTrGroups) {
+        // the issuing warp: the steps of the groups' tiles in turn
+        const bool issuer = tid == 0;
+        uint32_t parity = 0;
+        for (uint32_t t = 0; t < mine && ok; t += kTrGroups) {
+#pragma unroll 1
+            for (int step = 0; step < 8 && ok; step++) {
+#pragma unroll 1
+                for (uint32_t g = 0; g < (uint32_t)kTrGroups && t + g < mine && ok; g++) {
+                    const uint32_t ready = base + kTrMisc + 16 * g;
+                    const uint32_t tile = base + kImgBytes + kTrGroupBytes * g;
+                    const uint32_t d = tmem + 64u * g;
+                    const bool acc = t + g > 0;
+                    ok = __all_sync(0xffffffffu, wait_or_abort(ready, parity, abort));
+                    if (ok && issuer) {
+                        tc::fence_after_sync();
+                        const uint32_t h = tile + kTrH;
+                        if (step == 0) {
+                            gemm(d, Operand{tile + kTrX, kIn, false}, Operand{base + kImgW1, kIn, false}, kIn, kHid,
+                                 false);
+                        } else if (step < 4) {
+                            gemm(d, Operand{h + 16384u * (step - 1), kHid, false},
+                                 Operand{base + kImgW2 + 8192u * (step - 1), kHid, false}, kHid, kHid, false);
+                        } else if (step < 7) {
+                            // layer l's input gradient dY W and weight gradient A^T dY; dY of the output
+                            // layer in its own tile, else in the tile of the layer's activations
+                            const uint32_t l = 6u - (uint32_t)step;  // weights W(l + 2), input H(l + 1)
+                            const uint32_t dy = l == 2u ? tile + kTrDOut : h + 16384u * (l + 1u);
+                            const uint32_t cols = l == 2u ? (uint32_t)kGradOut : (uint32_t)kHid;
+                            gemm(d, Operand{dy, cols, false}, Operand{base + kImgW2 + 8192u * l, kHid, true},
+                                 (int)cols, kHid, false);
+                            gemm(grads + 64u * (l + 1u), Operand{h + 16384u * l, kHid, true},
+                                 Operand{dy, cols, true}, kRows, (int)cols, acc);
+                        } else {
+                            gemm(grads, Operand{tile + kTrX, kIn, true}, Operand{h, kHid, true}, kRows, kHid, acc);
+                        }
+                        tc::commit(ready + 8);
                     }
-                    float4* out = reinterpret_cast<float4*>(a.lobes + (size_t)row * kGuideLobeFloats);
-                    float f[40];
-#pragma unroll
-                    for (int k = 0; k < 8; k++) {
-                        const float mx = o[5 * k], my = o[5 * k + 1], mz = o[5 * k + 2];
-                        const float il = 1.f / (sqrtf(mx * mx + my * my + mz * mz) + 1e-6f);
-                        f[5 * k + 0] = mx * il;
-                        f[5 * k + 1] = my * il;
-                        f[5 * k + 2] = mz * il;
-                        f[5 * k + 3] = __expf(fminf(fmaxf(o[5 * k + 3], -3.f), 8.f));
-                        f[5 * k + 4] = e[k] / es;
-                    }
-#pragma unroll
-                    for (int i = 0; i < 10; i++) out[i] = make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]);
+                    __syncwarp();
                 }
-            } else {
-                float d[64];
-                const float l = mixture_grad(o, wdir, wt, d);
+                parity ^= 1u;
+            }
+        }
+        if (!ok && issuer) drain(base + kTrMisc + 128);
+        __syncwarp();
+    } else {
+        const uint32_t ready = base + kTrMisc + 16 * group, done = ready + 8;
+        const uint32_t lane_addr = tmem + 64u * group + ((uint32_t)(tid & ~31) << 16);
+        uint8_t* tile_sm = sm + kImgBytes + kTrGroupBytes * group;
+        const float w_scale = __ldg(a.w_scale);
+        uint32_t parity = 0;
+        auto step = [&]() {
+            arrive_ready(ready);
+            const bool got = __all_sync(0xffffffffu, wait_or_abort(done, parity, abort));
+            parity ^= 1u;
+            tc::fence_after_sync();
+            return got;
+        };
+        for (uint32_t t = group; t < mine && ok; t += kTrGroups) {
+            const uint32_t row = (blockIdx.x + t * gridDim.x) * kRows + tid;
+            const bool valid = row < n;
+            const Input x = load_input<true>(a, row, valid, w_scale);
+            store_features(tile_sm + kTrX, tid, x);
+            ok = step();
+#pragma unroll 1
+            for (int l = 0; l < 3 && ok; l++) {
+                float v[64];
+                load_row(lane_addr, v);
+                store_hidden(tile_sm + kTrH + 16384 * l, tid, v);
+                ok = step();
+            }
+            if (!ok) break;
+            {
+                float o[kGradOut], d[kGradOut];
+                load_row(lane_addr, o);
+                const float l = mixture_grad(o, x.wdir, x.wt, d);
                 if (valid) loss_sum += l;
 #pragma unroll
-                for (int c = 0; c < 8; c++) store_row8(R0 + 16384, tid, 8 * c, kOut, d + 8 * c);
-#pragma unroll
-                for (int j = 0; j < 64; j++) store_t(sm + kTrDT, j, tid, d[j]);
+                for (int c = 0; c < kGradOut / 8; c++)
+                    store_row8(tile_sm + kTrDOut, tid, 8 * c, kGradOut, d + 8 * c);
             }
-        }
-        if (TRAIN) {
-            const bool acc = done_tiles > 0;
-            // backward through layers 4, 3, 2: dH = (dY W) masked; dW^T += A^T dY
+            ok = step();
 #pragma unroll 1
-            for (int l = 2; l >= 0; l--) {
-                to_mma();
-                if (tid == 0) {
-                    tc::fence_after_sync();
-                    const uint32_t wt_img = base + (l == 2 ? kImgW4t : (l == 1 ? kImgW3t : kImgW2t));
-                    const uint32_t dy_rows = r0 + ((l & 1) ? 0u : 16384u);  // dOut in R0b, dH3 in R0a, dH2 in R0b
-                    gemm(tmem, dy_rows, wt_img, kOut, false);
-                    gemm(tmem + 128u + 64u * (uint32_t)l, base + kTrH1t + 16384u * (uint32_t)l, base + kTrDT, kRows,
-                         acc);
-                    tc::commit(mbar);
-                }
-                ok = wait_mma() && ok;
+            for (int l = 2; l >= 0 && ok; l--) {
                 float v[64];
-                load64(lane_addr, v);
-#pragma unroll
-                for (int j = 0; j < 64; j++) v[j] = ((mask[l][j >> 5] >> (j & 31)) & 1u) ? v[j] : 0.f;
-                if (l > 0) {
-                    uint8_t* dst = R0 + ((l & 1) ? 16384 : 0);
-#pragma unroll
-                    for (int c = 0; c < 8; c++) store_row8(dst, tid, 8 * c, kHid, v + 8 * c);
-                }
-#pragma unroll
-                for (int j = 0; j < 64; j++) store_t(sm + kTrDT, j, tid, v[j]);
+                load_row(lane_addr, v);
+                store_hidden_grad(tile_sm + kTrH + 16384 * l, tid, v);
+                ok = step();
             }
-            to_mma();
-            if (tid == 0) {
-                tc::fence_after_sync();
-                gemm(tmem + 64u, base + kTrXt, base + kTrDT, kRows, acc);
-                tc::commit(mbar);
-            }
-            ok = wait_mma() && ok;
-        }
-        done_tiles++;
-        if (__syncthreads_or(!ok)) {
-            if (tid == 0) atomicOr(a.err, 2);
-            break;
         }
     }
+    ok = !__syncthreads_or(!ok);
+    tc::fence_after_sync();
+    if (!ok && threadIdx.x == 0) atomicOr(a.err, 2);
 
-    if (TRAIN) {
-        // partial gradients of this CTA, in the parameter layout [out][in]
-        float* part = a.partials + (size_t)blockIdx.x * kGuideParams;
-        float v[64];
-        if (done_tiles > 0 && ok) {
-            load64(lane_addr + 64u, v);
+    // partial gradients of this CTA, in the parameter layout [out][in]
+    float* part = a.partials + (size_t)blockIdx.x * kGuideParams;
+    if (group == 0) {
+        if (mine > 0 && ok) {
+            const uint32_t lane_grads = grads + ((uint32_t)(tid & ~31) << 16);
+            float v[64];
+            load_row(lane_grads, v);
 #pragma unroll
             for (int j = 0; j < 64; j++) part[kW1 + j * kIn + tid] = v[j];
-            if (warp < 2) {
+            if (tid < kHid) {
 #pragma unroll 1
                 for (int l = 0; l < 3; l++) {
-                    load64(lane_addr + 128u + 64u * (uint32_t)l, v);
+                    load_row(lane_grads + 64u * (uint32_t)(l + 1), v);
                     const int off = l == 0 ? kW2 : (l == 1 ? kW3 : kW4);
 #pragma unroll
-                    for (int j = 0; j < 64; j++) part[off + j * kHid + tid] = v[j];
+                    for (int j = 0; j < 64; j++) part[off + j * kHid + tid] = l == 2 && j >= kGradOut ? 0.f : v[j];
                 }
             }
         } else {
             for (int i = tid; i < kGuideParams; i += kRows) part[i] = 0.f;
         }
+    }
+    if (group < kTrGroups) {
         float s = loss_sum;
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
@@ -457,7 +603,7 @@ __global__ void __launch_bounds__(kRows, 1) mlp_kernel(Mlp_Args a) {
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tmem, kCols);
+    if (threadIdx.x < 32) tc::tmem_dealloc(tmem, 512u);
 }
 
 // The MLP kernels' bounded mbarrier wait on a barrier that nothing arrives
@@ -472,7 +618,7 @@ __global__ void wait_selftest_kernel(uint32_t limit, int* err) {
     }
 }
 
-// fp32 parameters -> bf16 operand images (forward and transposed).
+// fp32 parameters -> bf16 operand images.
 __global__ void images_kernel(const float* __restrict__ params, uint8_t* __restrict__ img) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= kGuideParams) return;
@@ -488,9 +634,7 @@ __global__ void images_kernel(const float* __restrict__ params, uint8_t* __restr
     const int j = (i - kW2) % (kHid * kHid);
     const int nn = j / kHid, k = j % kHid;
     const uint32_t fwd = l == 0 ? kImgW2 : (l == 1 ? kImgW3 : kImgW4);
-    const uint32_t bwd = l == 0 ? kImgW2t : (l == 1 ? kImgW3t : kImgW4t);
     put(fwd + tc::tile_offset(nn, k, kHid));
-    put(bwd + tc::tile_offset(k, nn, kHid));
 }
 
 // Sum of the per-CTA partial gradients; Adam step when `lr` > 0, else the
@@ -501,6 +645,7 @@ __global__ void adam_kernel(const float* __restrict__ partials, int parts, float
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= kGuideParams) return;
     float g = 0.f;
+#pragma unroll 16
     for (int c = 0; c < parts; c++) g += partials[(size_t)c * kGuideParams + i];
     if (grad_out) {
         grad_out[i] = g;
@@ -543,10 +688,11 @@ int guide_ensure(yar_gpu_ctx* ctx) {
     static bool attr[64] = {};  // per device
     if (ctx->device < 0 || ctx->device >= 64) return fail(ctx, YAR_ERR_INVALID, "guide: device index");
     if (!attr[ctx->device]) {
-        e = cudaFuncSetAttribute(mlp_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrMisc + 64);
+        e = cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(kTrMisc + kMiscBytes));
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(mlp_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kInMisc + 64);
+            e = cudaFuncSetAttribute(mlp_infer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(kInMisc + kMiscBytes));
         if (e != cudaSuccess) return cuda_fail(ctx, e, "guide kernel attributes");
         attr[ctx->device] = true;
     }
@@ -604,8 +750,8 @@ cudaError_t guide_infer(yar_gpu_ctx* ctx, const float4* queries, uint32_t n_max,
     a.lobes = lobes;
     a.err = ctx->d_error;
     const uint32_t tiles = (n_max + kRows - 1) / kRows;
-    const uint32_t grid = std::min<uint32_t>(tiles, (uint32_t)sm_count() * 3u);  // 3 CTAs fit per SM
-    mlp_kernel<false><<<grid, kRows, kInMisc + 64, st>>>(a);
+    const uint32_t grid = std::min<uint32_t>(tiles, (uint32_t)sm_count());
+    mlp_infer_kernel<<<grid, kInThreads, kInMisc + kMiscBytes, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -630,7 +776,7 @@ cudaError_t guide_train(yar_gpu_ctx* ctx, const float4* samples, uint32_t n_max,
     a.err = ctx->d_error;
     const uint32_t tiles = (n_max + kRows - 1) / kRows;
     const int grid = (int)std::min<uint32_t>(tiles, (uint32_t)sm_count());
-    mlp_kernel<true><<<grid, kRows, kTrMisc + 64, st>>>(a);
+    mlp_train_kernel<<<grid, kTrThreads, kTrMisc + kMiscBytes, st>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     float c1 = 1.f, c2 = 1.f;
