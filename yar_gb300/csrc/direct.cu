@@ -378,7 +378,7 @@ direct_light_kernel(Render_Params p, Scene_Dev S, Direct_State D, const Direct_U
                 tmax = dist * (1.f - 1e-5f);
                 scale = n_dot_l / (dist * dist);
             }
-            if (ray) c = mul(col(dc.x, dc.y, dc.z) * bsdf_evaluate<true>(f, sc.wo, wi), scale);
+            if (ray) c = mul(col(dc.x, dc.y, dc.z) * bsdf_evaluate(f, sc.wo, wi), scale);
         } else {
             Col Le;
             float light_pdf = 0.f, ndw = 0.f;
@@ -422,10 +422,11 @@ direct_light_kernel(Render_Params p, Scene_Dev S, Direct_State D, const Direct_U
                 }
             }
             if (faces && ((ndw > 0.f && f.reflection) || (ndw < 0.f && f.transmission))) {
-                const Col fv = bsdf_evaluate<true>(f, sc.wo, wi);
+                float bpdf;
+                const Col fv = bsdf_value(f, sc.wo, wi, bpdf);
                 if (!black(fv)) {
                     ray = true;
-                    const float w = mis_power(light_pdf, bsdf_pdf<true>(f, sc.wo, wi));
+                    const float w = mis_power(light_pdf, bpdf);
                     c = mul(Le * fv, w * fabsf(ndw) / light_pdf);
                 }
             }
@@ -468,27 +469,36 @@ direct_bsdf_kernel(Render_Params p, Scene_Dev S, Direct_State D, const Direct_Un
                                     __ldg(s1d + ((size_t)lp * p.n1d + u.grid1 + u.element) * p.spp + sample)) *
                                    (1.f / (float)u.count));
         }
-        float bpdf = 0.f;
-        const Col fv = bsdf_sample<true>(f, ub.x, ub.y, us, sc.wo, wi, bpdf);
-        float lndw = 1.f;
+        Bsdf_Sample bs;
+        const bool alive = bsdf_direction(f, ub.x, ub.y, us, sc.wo, bs);
+        wi = bs.wi;
+        float bpdf = 0.f, lndw = 1.f;
         float4 probe = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (!black(fv)) {
-            if (u.kind == kUnitRect) {
-                const Rect_Light_Dev& T = S.lights[u.light];
+        // towards the light, then the value: most samples go elsewhere
+        if (alive && u.kind == kUnitRect) {
+            const Rect_Light_Dev& T = S.lights[u.light];
+            lndw = dot(v3(__ldg(&T.r0).z, __ldg(&T.r1).z, __ldg(&T.r2).z), -wi);
+            if (lndw > 1e-4f) {
+                const Col fv = bsdf_sampled_value(f, sc.wo, bs, bpdf);
                 const float4 le = __ldg(&T.le);
-                lndw = dot(v3(__ldg(&T.r0).z, __ldg(&T.r1).z, __ldg(&T.r2).z), -wi);
-                ray = lndw > 1e-4f;
                 const Col c = col(le.x, le.y, le.z) * fv;
+                ray = !black(fv);
                 probe = make_float4(c.r, c.g, c.b, bpdf);
-            } else if (u.kind == kUnitSphere) {
-                const float4 sa = __ldg(&S.sphere_lights[u.light].a), le = __ldg(&S.sphere_lights[u.light].le);
-                Sphere_Sampler ss;
-                sphere_sampler_init(ss, v3(sa.x, sa.y, sa.z), sa.w, sc.position);
-                ray = dot(-ss.axes[2], wi) >= ss.cos_theta_max;
+            }
+        } else if (alive && u.kind == kUnitSphere) {
+            const float4 sa = __ldg(&S.sphere_lights[u.light].a), le = __ldg(&S.sphere_lights[u.light].le);
+            Sphere_Sampler ss;
+            sphere_sampler_init(ss, v3(sa.x, sa.y, sa.z), sa.w, sc.position);
+            if (dot(-ss.axes[2], wi) >= ss.cos_theta_max) {
+                const Col fv = bsdf_sampled_value(f, sc.wo, bs, bpdf);
                 const float w = mis_power(bpdf, ss.cone_pdf);
                 const Col c = mul(col(le.x, le.y, le.z) * fv, w * fabsf(dot(sc.n, wi)) / bpdf);
+                ray = !black(fv);
                 probe = make_float4(c.r, c.g, c.b, 0.f);
-            } else {
+            }
+        } else if (alive) {
+            const Col fv = bsdf_sampled_value(f, sc.wo, bs, bpdf);
+            if (!black(fv)) {
                 const Col Le = env_radiance(S, wi, false);
                 ray = !black(Le);
                 const float w = mis_power(bpdf, env_light_pdf(S, wi));

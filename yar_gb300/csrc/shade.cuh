@@ -563,38 +563,12 @@ __device__ __forceinline__ float pow5(float v) { return (v * v) * (v * v) * v; }
 
 // The FULL forms (every material, mixes included) are called out of line:
 // inlined at each of the shade kernels' call sites they multiplied the
-// kernels' code and took the device compiler minutes per kernel.  The
-// FULL = false forms (diffuse, metal, rough glass) stay inlined.
-template <bool FULL> __device__ __forceinline__ Col leaf_evaluate_body(const Bsdf& f, V3 wo, V3 wi);
-template <bool FULL> __device__ __forceinline__ float leaf_pdf_body(const Bsdf& f, V3 wo, V3 wi);
-template <bool FULL>
-__device__ __forceinline__ Col leaf_sample_body(const Bsdf& f, float u0, float u1, float u_scatter, V3 wo, V3& wi,
-                                                float& pdf);
-static __device__ __noinline__ Col leaf_evaluate_full(const Bsdf& f, V3 wo, V3 wi) { return leaf_evaluate_body<true>(f, wo, wi); }
-static __device__ __noinline__ float leaf_pdf_full(const Bsdf& f, V3 wo, V3 wi) { return leaf_pdf_body<true>(f, wo, wi); }
-static __device__ __noinline__ Col leaf_sample_full(const Bsdf& f, float u0, float u1, float u_scatter, V3 wo, V3& wi,
-                                             float& pdf) {
-    return leaf_sample_body<true>(f, u0, u1, u_scatter, wo, wi, pdf);
-}
-template <bool FULL = true>
-__device__ __forceinline__ Col leaf_evaluate(const Bsdf& f, V3 wo, V3 wi) {
-    if constexpr (FULL) return leaf_evaluate_full(f, wo, wi);
-    else return leaf_evaluate_body<false>(f, wo, wi);
-}
-template <bool FULL = true>
-__device__ __forceinline__ float leaf_pdf(const Bsdf& f, V3 wo, V3 wi) {
-    if constexpr (FULL) return leaf_pdf_full(f, wo, wi);
-    else return leaf_pdf_body<false>(f, wo, wi);
-}
-template <bool FULL = true>
-__device__ __forceinline__ Col leaf_sample(const Bsdf& f, float u0, float u1, float u_scatter, V3 wo, V3& wi,
-                                           float& pdf) {
-    if constexpr (FULL) return leaf_sample_full(f, u0, u1, u_scatter, wo, wi, pdf);
-    else return leaf_sample_body<false>(f, u0, u1, u_scatter, wo, wi, pdf);
-}
+// kernels' code and took the device compiler minutes per kernel.  The plain
+// materials (diffuse, metal, rough glass) have their value and density in one
+// routine (plain_value).
+static __device__ __noinline__ Col leaf_evaluate(const Bsdf& f, V3 wo, V3 wi);
+static __device__ __noinline__ float leaf_pdf(const Bsdf& f, V3 wo, V3 wi);
 
-// FULL = false compiles out the plastic and coated-diffuse branches, for
-// scenes that only use the diffuse, metal and rough-glass BSDFs.
 // cos_delta_phi (src/lib/math.h:87-104): the cosine of the azimuth between a
 // and b in the tangent plane (1 for a direction along the normal).
 __device__ __forceinline__ float cos_delta_phi(V3 a, V3 b, V3 t1, V3 t2) {
@@ -654,11 +628,10 @@ static __device__ __noinline__ Col fourier_evaluate(const Bsdf& f, V3 wo, V3 wi)
     return col(r * scale, g * scale, b * scale);
 }
 
-template <bool FULL>
-__device__ __forceinline__ Col leaf_evaluate_body(const Bsdf& f, V3 wo, V3 wi) {
+static __device__ __noinline__ Col leaf_evaluate(const Bsdf& f, V3 wo, V3 wi) {
     if (f.type == kDiffuse) return mul(f.reflectance, 1.f / kPi);
-    if (FULL && f.type == kFourier) return fourier_evaluate(f, wo, wi);
-    if (FULL && (f.type == kPlastic || f.type == kPbrt3Plastic)) {
+    if (f.type == kFourier) return fourier_evaluate(f, wo, wi);
+    if (f.type == kPlastic || f.type == kPbrt3Plastic) {
         // Plastic_BRDF::evaluate (src/ref/bsdf.cpp:215-234); Pbrt3_Plastic_BRDF::evaluate
         // (src/ref/bsdf_pbrt.cpp:264-290) with pbrt-v3's swapped 1.0 / 1.5 IOR pair
         const V3 wh = normalized(wo + wi);
@@ -676,11 +649,11 @@ __device__ __forceinline__ Col leaf_evaluate_body(const Bsdf& f, V3 wo, V3 wi) {
         const Col base = mul(F, (G * D) / (4.f * dot(wo, f.n) * dot(wi, f.n)));
         return mul(f.reflectance, 1.f / kPi) + mul(base, f.transmittance.r);
     }
-    if (FULL && f.type == kDiffuseTransmission) {  // Diffuse_Transmission_BSDF::evaluate (bsdf.cpp:105-112)
+    if (f.type == kDiffuseTransmission) {  // Diffuse_Transmission_BSDF::evaluate (bsdf.cpp:105-112)
         const bool same = dot(wo, f.n) * dot(wi, f.n) > 0.f;
         return mul(same ? f.reflectance : f.transmittance, 1.f / kPi);
     }
-    if (FULL && f.type == kUber) {  // Pbrt3_Uber_BRDF::evaluate (bsdf_pbrt.cpp:34-52)
+    if (f.type == kUber) {  // Pbrt3_Uber_BRDF::evaluate (bsdf_pbrt.cpp:34-52)
         const Col diffuse = mul(f.reflectance, 1.f / kPi) * f.extra;
         const V3 wo_l = world_to_local(f, wo), wi_l = world_to_local(f, wi);
         const V3 wh_l = normalized(wo_l + wi_l);
@@ -690,7 +663,7 @@ __device__ __forceinline__ Col leaf_evaluate_body(const Bsdf& f, V3 wo, V3 wi) {
         const float m = (F * G * D) / (4.f * wo_l.z * wi_l.z);
         return diffuse + mul(f.specular * f.extra, m);
     }
-    if (FULL && f.type == kTranslucent) {  // Pbrt3_Translucent_BSDF::evaluate (bsdf_pbrt.cpp:117-158)
+    if (f.type == kTranslucent) {  // Pbrt3_Translucent_BSDF::evaluate (bsdf_pbrt.cpp:117-158)
         if (dot(wo, f.n) * dot(wi, f.n) > 0.f) {
             const Col diffuse = mul(f.extra, 1.f / kPi) * f.reflectance;
             const V3 wh = normalized(wo + wi);
@@ -718,7 +691,7 @@ __device__ __forceinline__ Col leaf_evaluate_body(const Bsdf& f, V3 wo, V3 wi) {
         }
         return diffuse + specular;
     }
-    if (FULL && f.type == kCoatedDiffuse) {
+    if (f.type == kCoatedDiffuse) {
         // Ashikhmin_Shirley_Phong_BRDF::evaluate (src/ref/bsdf.cpp:440-460)
         const V3 wo_l = world_to_local(f, wo), wi_l = world_to_local(f, wi);
         const V3 wh_l = normalized(wo_l + wi_l);
@@ -765,29 +738,28 @@ __device__ __forceinline__ Col leaf_evaluate_body(const Bsdf& f, V3 wo, V3 wi) {
     return mul(f.transmittance, base);
 }
 
-template <bool FULL>
-__device__ __forceinline__ float leaf_pdf_body(const Bsdf& f, V3 wo, V3 wi) {
+static __device__ __noinline__ float leaf_pdf(const Bsdf& f, V3 wo, V3 wi) {
     // Pbrt3_Fourier_BSDF::pdf (src/ref/bsdf_pbrt.cpp:368-372): cosine-weighted as diffuse
-    if (f.type == kDiffuse || (FULL && f.type == kFourier)) return dot(f.n, wi) / kPi;
-    if (FULL && (f.type == kPlastic || f.type == kPbrt3Plastic)) {  // Plastic_BRDF::pdf (src/ref/bsdf.cpp:253-263)
+    if (f.type == kDiffuse || f.type == kFourier) return dot(f.n, wi) / kPi;
+    if (f.type == kPlastic || f.type == kPbrt3Plastic) {  // Plastic_BRDF::pdf (src/ref/bsdf.cpp:253-263)
         const float diffuse_pdf = dot(f.n, wi) / kPi;
         const V3 wh = normalized(wo + wi);
         const float spec_pdf = vndf_pdf(wo, wh, f.n, f.alpha) / (4 * dot(wh, wo));
         return 0.5f * (diffuse_pdf + spec_pdf);
     }
-    if (FULL && f.type == kDiffuseTransmission) {  // Diffuse_Transmission_BSDF::pdf (bsdf.cpp:128-141)
+    if (f.type == kDiffuseTransmission) {  // Diffuse_Transmission_BSDF::pdf (bsdf.cpp:128-141)
         const float max_r = max_component(f.reflectance), max_t = max_component(f.transmittance);
         const float pdf = fabsf(dot(f.n, wi)) * (1.f / kPi);
         return dot(wo, f.n) * dot(wi, f.n) > 0.f ? (max_r / (max_r + max_t)) * pdf : (max_t / (max_r + max_t)) * pdf;
     }
-    if (FULL && f.type == kUber) {  // Pbrt3_Uber_BRDF::pdf (bsdf_pbrt.cpp:74-87)
+    if (f.type == kUber) {  // Pbrt3_Uber_BRDF::pdf (bsdf_pbrt.cpp:74-87)
         const float diffuse_pdf = dot(f.n, wi) / kPi;
         const V3 wo_l = world_to_local(f, wo), wi_l = world_to_local(f, wi);
         const V3 wh_l = normalized(wo_l + wi_l);
         const float spec_pdf = vndf_pdf_aniso(wo_l, wh_l, f.alpha_x, f.alpha_y) / (4 * dot(wh_l, wo_l));
         return 0.5f * (diffuse_pdf + spec_pdf);
     }
-    if (FULL && f.type == kTranslucent) {  // Pbrt3_Translucent_BSDF::pdf (bsdf_pbrt.cpp:211-250)
+    if (f.type == kTranslucent) {  // Pbrt3_Translucent_BSDF::pdf (bsdf_pbrt.cpp:211-250)
         const float max_r = max_component(f.reflectance), max_t = max_component(f.transmittance);
         const float rp = max_r / (max_r + max_t);
         if (dot(wo, f.n) * dot(wi, f.n) > 0.f) {
@@ -807,7 +779,7 @@ __device__ __forceinline__ float leaf_pdf_body(const Bsdf& f, V3 wo, V3 wi) {
         }
         return (1.f - rp) * 0.5f * (diffuse_pdf + spec_pdf);
     }
-    if (FULL && f.type == kCoatedDiffuse) {  // Ashikhmin_Shirley_Phong_BRDF::pdf (src/ref/bsdf.cpp:480-492)
+    if (f.type == kCoatedDiffuse) {  // Ashikhmin_Shirley_Phong_BRDF::pdf (src/ref/bsdf.cpp:480-492)
         const float diffuse_pdf = dot(f.n, wi) / kPi;
         const V3 wo_l = world_to_local(f, wo), wi_l = world_to_local(f, wi);
         const V3 wh_l = normalized(wo_l + wi_l);
@@ -838,16 +810,77 @@ __device__ __forceinline__ float leaf_pdf_body(const Bsdf& f, V3 wo, V3 wi) {
     return (wh_pdf * dwh) * (1.f - rprob);
 }
 
-// BSDF::sample; black when no direction is produced.
+// The value and density of the plain materials (the expressions of
+// leaf_evaluate and leaf_pdf above, what they share computed once).  For a
+// metal's own sample (`sampled`) the density takes the microfacet normal wh
+// (local frame) that was drawn, not the one between wo and wi.
+// The shade kernel is bound by its instructions, a quarter of them divisions.
+// The GGX room, 512 x 512 samples of 64, in full: 42.2 ms with value and
+// density computed apart and the whole BSDF sample taken before asking whether
+// its probe may reach the light; 41.0 ms as below but out of line, 40.2 ms
+// inlined at its three call sites (the BSDF then stays in registers).
+__device__ __forceinline__ Col plain_value(const Bsdf& f, V3 wo, V3 wi, bool sampled, V3 wh, float& pdf) {
+    if (f.type == kDiffuse) {
+        pdf = dot(f.n, wi) / kPi;
+        return mul(f.reflectance, 1.f / kPi);
+    }
+    if (f.type == kMetal) {
+        const V3 wo_l = world_to_local(f, wo), wi_l = world_to_local(f, wi);
+        const V3 wh_l = normalized(wo_l + wi_l);
+        const float lambda_o = ggx_lambda_aniso(wo_l, f.alpha_x, f.alpha_y);
+        const float G = 1.f / (1.f + ggx_lambda_aniso(wi_l, f.alpha_x, f.alpha_y) + lambda_o);
+        const float D = ggx_D_aniso(wh_l, f.alpha_x, f.alpha_y);
+        if (!sampled) wh = wh_l;
+        const float D_wh = sampled ? ggx_D_aniso(wh, f.alpha_x, f.alpha_y) : D;
+        const float G1 = 1.f / (1.f + lambda_o);
+        pdf = G1 * D_wh * max_std(0.f, dot(wo_l, wh)) / wo_l.z / (4 * dot(wh, wo_l));
+        const Col F = conductor_fresnel(dot(wi_l, wh_l), f.eta_i_metal, f.eta_t, f.k_t);
+        return mul(F, (G * D) / (4.f * wo_l.z * wi_l.z));
+    }
+    const float wo_n = dot(wo, f.n), wi_n = dot(wi, f.n);
+    const bool same = wo_n * wi_n > 0.f;
+    const V3 h = same ? normalized(wo + wi) : refraction_half(f.eta_o, wo, f.eta_i, wi, f.n);
+    const float wo_wh = dot(wo, h), wi_wh = dot(wi, h);
+    pdf = 0.f;
+    if (!same && wo_wh * wi_wh > 0.f) return col(0.f, 0.f, 0.f);
+    const float lambda_o = ggx_lambda(wo, f.n, f.alpha);
+    const float G = 1.f / (1.f + ggx_lambda(wi, f.n, f.alpha) + lambda_o);
+    const float D = ggx_D(h, f.n, f.alpha);
+    const float h_pdf = 1.f / (1.f + lambda_o) * D * max_std(0.f, wo_wh) / wo_n;
+    const float F = dielectric_fresnel(wi_wh, same ? f.eta_i / f.eta_o : f.eta_o / f.eta_i);
+    if (same) {
+        pdf = h_pdf / (4 * wo_wh) * glass_reflection_probability(f, F);
+        if (sampled && pdf == 0.f) return col(0.f, 0.f, 0.f);
+        return mul(f.reflectance, (F * G * D) / (4.f * wo_n * wi_n));
+    }
+    const float k2 = f.eta_o * wo_wh + f.eta_i * wi_wh;
+    const float rprob = glass_reflection_probability(f, dielectric_fresnel(wo_wh, f.eta_i / f.eta_o));
+    pdf = (h_pdf * (f.eta_i * f.eta_i * fabsf(wi_wh) / (k2 * k2))) * (1.f - rprob);
+    if ((sampled && pdf == 0.f) || F == 1.f) return col(0.f, 0.f, 0.f);
+    const float k = fabsf((wo_wh * wi_wh) / (wo_n * wi_n));
+    return mul(f.transmittance, (f.eta_o * f.eta_o * k * G * D * (1.f - F)) / (k2 * k2));
+}
+
+// BSDF::sample in two steps: the direction, then (where the caller still
+// wants it) its value and density.  A light's BSDF sample only counts if its
+// direction may reach the light, which most do not.
+struct Bsdf_Sample {
+    V3 wi;  // the zero vector (the reference's default-constructed direction) where a leaf gave up early
+    V3 wh;  // metal: the microfacet normal drawn
+    bool ok;      // the leaf produced a direction
+    bool second;  // mix: the leaf was the second material
+};
 template <bool FULL>
-__device__ __forceinline__ Col leaf_sample_body(const Bsdf& f, float u0, float u1, float u_scatter, V3 wo, V3& wi,
-                                                float& pdf) {
+__device__ __forceinline__ Bsdf_Sample leaf_direction(const Bsdf& f, float u0, float u1, float u_scatter, V3 wo) {
+    Bsdf_Sample r;
+    r.wi = r.wh = v3(0.f, 0.f, 0.f);
+    r.ok = r.second = false;
     if (FULL && f.type == kDiffuseTransmission) {  // Diffuse_Transmission_BSDF::sample (bsdf.cpp:114-126)
         const float max_r = max_component(f.reflectance), max_t = max_component(f.transmittance);
         const float sign = u_scatter < max_r / (max_r + max_t) ? 1.f : -1.f;
-        wi = local_to_world(f, mul(sample_hemisphere_cosine(u0, u1), sign));
-        pdf = leaf_pdf<FULL>(f, wo, wi);
-        return leaf_evaluate<FULL>(f, wo, wi);
+        r.wi = local_to_world(f, mul(sample_hemisphere_cosine(u0, u1), sign));
+        r.ok = true;
+        return r;
     }
     if (FULL && f.type == kTranslucent) {  // Pbrt3_Translucent_BSDF::sample (bsdf_pbrt.cpp:160-209)
         const float max_r = max_component(f.reflectance), max_t = max_component(f.transmittance);
@@ -856,183 +889,194 @@ __device__ __forceinline__ Col leaf_sample_body(const Bsdf& f, float u0, float u
         const float u = one_minus_eps_min_s(reflect_side ? u_scatter / rp : (u_scatter - rp) / (1.f - rp));
         if (u < 0.5f) {
             const V3 l = sample_hemisphere_cosine(u0, u1);
-            wi = local_to_world(f, reflect_side ? l : -l);
+            r.wi = local_to_world(f, reflect_side ? l : -l);
         } else {
             const V3 wh = local_to_world(f, ggx_sample_vndf(u0, u1, world_to_local(f, wo), f.alpha, f.alpha));
+            V3 c;
             if (reflect_side) {
-                const V3 c = reflect(wo, wh);
-                if (dot(c, f.n) <= 0.f) return col(0.f, 0.f, 0.f);
-                wi = c;
+                c = reflect(wo, wh);
+                if (dot(c, f.n) <= 0.f) return r;
             } else {
-                if (dot(wh, wo) < 0.f) return col(0.f, 0.f, 0.f);
-                V3 c;
-                if (!refract(wo, wh, f.eta_o / f.eta_i, c)) return col(0.f, 0.f, 0.f);
-                if (dot(c, f.n) >= 0.f) return col(0.f, 0.f, 0.f);
-                wi = c;
+                if (dot(wh, wo) < 0.f) return r;
+                if (!refract(wo, wh, f.eta_o / f.eta_i, c)) return r;
+                if (dot(c, f.n) >= 0.f) return r;
             }
+            r.wi = c;
         }
-        pdf = leaf_pdf<FULL>(f, wo, wi);
-        if (pdf == 0.f) return col(0.f, 0.f, 0.f);
-        return leaf_evaluate<FULL>(f, wo, wi);
+        r.ok = true;
+        return r;
     }
     if (FULL && (f.type == kPlastic || f.type == kPbrt3Plastic || f.type == kCoatedDiffuse || f.type == kUber)) {
         // Plastic_BRDF::sample (src/ref/bsdf.cpp:236-251), Ashikhmin_Shirley_Phong_BRDF::sample
         // (:462-478): the first 1D sample picks the diffuse or the specular lobe
         if (u_scatter < 0.5f) {
-            wi = local_to_world(f, sample_hemisphere_cosine(u0, u1));
+            r.wi = local_to_world(f, sample_hemisphere_cosine(u0, u1));
         } else {
             const V3 wo_l = world_to_local(f, wo);
             if (f.type == kCoatedDiffuse || f.type == kUber) {
                 const V3 wh_l = ggx_sample_vndf(u0, u1, wo_l, f.alpha_x, f.alpha_y);
-                wi = local_to_world(f, reflect(wo_l, wh_l));
+                r.wi = local_to_world(f, reflect(wo_l, wh_l));
             } else {
                 const V3 wh = local_to_world(f, ggx_sample_vndf(u0, u1, wo_l, f.alpha, f.alpha));
-                wi = reflect(wo, wh);
+                r.wi = reflect(wo, wh);
             }
         }
-        if (dot(f.n, wi) <= 0.f) return col(0.f, 0.f, 0.f);
-        pdf = leaf_pdf<FULL>(f, wo, wi);
-        return leaf_evaluate<FULL>(f, wo, wi);
+        r.ok = !(dot(f.n, r.wi) <= 0.f);
+        return r;
     }
     if (f.type == kDiffuse || (FULL && f.type == kFourier)) {  // Pbrt3_Fourier_BSDF::sample: as diffuse
-        wi = local_to_world(f, sample_hemisphere_cosine(u0, u1));
-        pdf = leaf_pdf<FULL>(f, wo, wi);
-        return leaf_evaluate<FULL>(f, wo, wi);
-    }
-    if (f.type == kMetal) {
-        const V3 wo_l = world_to_local(f, wo);
-        const V3 wh_l = ggx_sample_vndf(u0, u1, wo_l, f.alpha_x, f.alpha_y);
-        const V3 wi_l = reflect(wo_l, wh_l);
-        if (wi_l.z <= 0.f) return col(0.f, 0.f, 0.f);
-        wi = local_to_world(f, wi_l);
-        pdf = vndf_pdf_aniso(wo_l, wh_l, f.alpha_x, f.alpha_y) / (4 * dot(wh_l, wo_l));
-        return leaf_evaluate<FULL>(f, wo, wi);
+        r.wi = local_to_world(f, sample_hemisphere_cosine(u0, u1));
+        r.ok = true;
+        return r;
     }
     const V3 wo_l = world_to_local(f, wo);
+    if (f.type == kMetal) {
+        r.wh = ggx_sample_vndf(u0, u1, wo_l, f.alpha_x, f.alpha_y);
+        const V3 wi_l = reflect(wo_l, r.wh);
+        if (wi_l.z <= 0.f) return r;
+        r.wi = local_to_world(f, wi_l);
+        r.ok = true;
+        return r;
+    }
     const V3 wh = local_to_world(f, ggx_sample_vndf(u0, u1, wo_l, f.alpha, f.alpha));
     const V3 rwi = reflect(wo, wh);
-    if (dot(rwi, f.n) <= 0.f) return col(0.f, 0.f, 0.f);
+    if (dot(rwi, f.n) <= 0.f) return r;
     const float fresnel = dielectric_fresnel(dot(wo, wh), f.eta_i / f.eta_o);
     const float rprob = glass_reflection_probability(f, fresnel);
     if (u_scatter < rprob) {
-        wi = rwi;
+        r.wi = rwi;
     } else {
-        if (!refract(wo, wh, f.eta_o / f.eta_i, wi)) return col(0.f, 0.f, 0.f);
-        if (dot(wi, f.n) >= 0.f) return col(0.f, 0.f, 0.f);
+        V3 c = v3(0.f, 0.f, 0.f);
+        const bool refracted = refract(wo, wh, f.eta_o / f.eta_i, c);
+        r.wi = c;
+        if (!refracted || dot(c, f.n) >= 0.f) return r;
     }
-    pdf = leaf_pdf<FULL>(f, wo, wi);
-    if (pdf == 0.f) return col(0.f, 0.f, 0.f);
-    return leaf_evaluate<FULL>(f, wo, wi);
+    r.ok = true;
+    return r;
+}
+__device__ __forceinline__ bool plain_material(const Bsdf& f) {
+    return f.type == kDiffuse || f.type == kMetal || f.type == kGlass;
+}
+// The value of a leaf's own sample, black where its sampling gives up.
+static __device__ __noinline__ Col leaf_sampled_value(const Bsdf& f, V3 wo, const Bsdf_Sample& s, float& pdf) {
+    if (plain_material(f)) return plain_value(f, wo, s.wi, true, s.wh, pdf);
+    pdf = leaf_pdf(f, wo, s.wi);
+    if (f.type == kTranslucent && pdf == 0.f) return col(0.f, 0.f, 0.f);
+    return leaf_evaluate(f, wo, s.wi);
+}
+static __device__ __noinline__ Col leaf_value(const Bsdf& f, V3 wo, V3 wi, float& pdf) {
+    if (plain_material(f)) return plain_value(f, wo, wi, false, wi, pdf);
+    pdf = leaf_pdf(f, wo, wi);
+    return leaf_evaluate(f, wo, wi);
 }
 
 // Mix_BSDF (src/ref/bsdf.cpp:497-567) and Scaled_BSDF (:572-592) over leaf BSDFs;
-// every other BSDF forwards.  FULL = false compiles the mix out.
+// every other BSDF forwards.
 __device__ __forceinline__ bool possible_for(const Bsdf& f, float n_dot_wi) {
     return (n_dot_wi > 0.f && f.reflection) || (n_dot_wi < 0.f && f.transmission);
 }
-template <bool FULL>
-__device__ __forceinline__ Col bsdf_evaluate_body(const Bsdf& f, V3 wo, V3 wi) {
-    if (FULL && f.type == kScaled) {
+// Only the value (point, spot and directional lights, of scenes that need the FULL forms).
+static __device__ __noinline__ Col bsdf_evaluate(const Bsdf& f, V3 wo, V3 wi) {
+    if (f.type == kScaled) {
         Bsdf a = f;
         set_material(a, *f.sub[0]);
-        return mul(leaf_evaluate<true>(a, wo, wi), f.mix_p);
+        return mul(leaf_evaluate(a, wo, wi), f.mix_p);
     }
-    if (FULL && f.type == kMix) {
+    if (f.type == kMix) {
         Bsdf a = f, b = f;
         set_material(a, *f.sub[0]);
         set_material(b, *f.sub[1]);
         Col f1 = col(0.f, 0.f, 0.f), f2 = col(0.f, 0.f, 0.f);
         const float n_dot_wi = dot(f.n, wi);
-        if (possible_for(a, n_dot_wi)) f1 = leaf_evaluate<true>(a, wo, wi);
-        if (possible_for(b, n_dot_wi)) f2 = leaf_evaluate<true>(b, wo, wi);
+        if (possible_for(a, n_dot_wi)) f1 = leaf_evaluate(a, wo, wi);
+        if (possible_for(b, n_dot_wi)) f2 = leaf_evaluate(b, wo, wi);
         return (col(1.f, 1.f, 1.f) - f.mix_coeff) * f1 + f.mix_coeff * f2;
     }
-    return leaf_evaluate<FULL>(f, wo, wi);
+    return leaf_evaluate(f, wo, wi);
 }
-template <bool FULL>
-__device__ __forceinline__ float bsdf_pdf_body(const Bsdf& f, V3 wo, V3 wi) {
-    if (FULL && f.type == kScaled) {
+static __device__ __noinline__ Col bsdf_value_full(const Bsdf& f, V3 wo, V3 wi, float& pdf) {
+    if (f.type == kScaled) {
         Bsdf a = f;
         set_material(a, *f.sub[0]);
-        return leaf_pdf<true>(a, wo, wi);
+        return mul(leaf_value(a, wo, wi, pdf), f.mix_p);
     }
-    if (FULL && f.type == kMix) {
-        Bsdf a = f, b = f;
-        set_material(a, *f.sub[0]);
-        set_material(b, *f.sub[1]);
-        float pdf1 = 0.f, pdf2 = 0.f;
-        const float n_dot_wi = dot(f.n, wi);
-        if (possible_for(a, n_dot_wi)) pdf1 = leaf_pdf<true>(a, wo, wi);
-        if (possible_for(b, n_dot_wi)) pdf2 = leaf_pdf<true>(b, wo, wi);
-        return (1.f - f.mix_p) * pdf1 + f.mix_p * pdf2;
-    }
-    return leaf_pdf<FULL>(f, wo, wi);
-}
-// wi must come in as the zero vector: the reference's default-constructed
-// direction, which a leaf sample that gives up early leaves as it is.
-template <bool FULL>
-__device__ __forceinline__ Col bsdf_sample_body(const Bsdf& f, float u0, float u1, float u_scatter, V3 wo, V3& wi,
-                                                float& pdf) {
-    if (FULL && f.type == kScaled) {
-        Bsdf a = f;
-        set_material(a, *f.sub[0]);
-        return mul(leaf_sample<true>(a, u0, u1, u_scatter, wo, wi, pdf), f.mix_p);
-    }
-    if (FULL && f.type == kMix) {
+    if (f.type == kMix) {
         Bsdf a = f, b = f;
         set_material(a, *f.sub[0]);
         set_material(b, *f.sub[1]);
         Col f1 = col(0.f, 0.f, 0.f), f2 = col(0.f, 0.f, 0.f);
         float pdf1 = 0.f, pdf2 = 0.f;
-        if (u_scatter < f.mix_p) {
-            f2 = leaf_sample<true>(b, u0, u1, u_scatter / f.mix_p, wo, wi, pdf2);
-            if (possible_for(a, dot(f.n, wi))) {
-                pdf1 = leaf_pdf<true>(a, wo, wi);
-                f1 = leaf_evaluate<true>(a, wo, wi);
-            }
-        } else {
-            f1 = leaf_sample<true>(a, u0, u1, (u_scatter - f.mix_p) / (1.f - f.mix_p), wo, wi, pdf1);
-            if (possible_for(b, dot(f.n, wi))) {
-                pdf2 = leaf_pdf<true>(b, wo, wi);
-                f2 = leaf_evaluate<true>(b, wo, wi);
-            }
-        }
+        const float n_dot_wi = dot(f.n, wi);
+        if (possible_for(a, n_dot_wi)) f1 = leaf_value(a, wo, wi, pdf1);
+        if (possible_for(b, n_dot_wi)) f2 = leaf_value(b, wo, wi, pdf2);
         pdf = (1.f - f.mix_p) * pdf1 + f.mix_p * pdf2;
         return (col(1.f, 1.f, 1.f) - f.mix_coeff) * f1 + f.mix_coeff * f2;
     }
-    return leaf_sample<FULL>(f, u0, u1, u_scatter, wo, wi, pdf);
+    return leaf_value(f, wo, wi, pdf);
 }
-
-static __device__ __noinline__ Col bsdf_evaluate_full(const Bsdf& f, V3 wo, V3 wi) { return bsdf_evaluate_body<true>(f, wo, wi); }
-static __device__ __noinline__ float bsdf_pdf_full(const Bsdf& f, V3 wo, V3 wi) { return bsdf_pdf_body<true>(f, wo, wi); }
-static __device__ __noinline__ Col bsdf_sample_full(const Bsdf& f, float u0, float u1, float u_scatter, V3 wo, V3& wi,
-                                             float& pdf) {
-    return bsdf_sample_body<true>(f, u0, u1, u_scatter, wo, wi, pdf);
+static __device__ __noinline__ Bsdf_Sample bsdf_direction_full(const Bsdf& f, float u0, float u1, float u_scatter,
+                                                               V3 wo) {
+    if (f.type == kScaled || f.type == kMix) {
+        const bool second = f.type == kMix && u_scatter < f.mix_p;
+        if (f.type == kMix) u_scatter = second ? u_scatter / f.mix_p : (u_scatter - f.mix_p) / (1.f - f.mix_p);
+        Bsdf a = f;
+        set_material(a, *f.sub[second ? 1 : 0]);
+        Bsdf_Sample s = leaf_direction<true>(a, u0, u1, u_scatter, wo);
+        s.second = second;
+        return s;
+    }
+    return leaf_direction<true>(f, u0, u1, u_scatter, wo);
 }
-// The plain (diffuse, metal, rough glass) sampling routine is called out of
-// line too: the shade kernel calls it at two places, and its stalls are mostly
-// instruction fetch (ncu: 29.6 cycles of no_instruction per issue).  C3 render
-// on GB300: 1.546 s against 1.598 s inlined; evaluation out of line as well
-// measured 1.565 s.
-static __device__ __noinline__ Col bsdf_sample_plain(const Bsdf& f, float u0, float u1, float u_scatter, V3 wo,
-                                                     V3& wi, float& pdf) {
-    return bsdf_sample_body<false>(f, u0, u1, u_scatter, wo, wi, pdf);
+static __device__ __noinline__ Col bsdf_sampled_value_full(const Bsdf& f, V3 wo, const Bsdf_Sample& s, float& pdf) {
+    if (f.type == kScaled) {
+        Bsdf a = f;
+        set_material(a, *f.sub[0]);
+        return mul(leaf_sampled_value(a, wo, s, pdf), f.mix_p);
+    }
+    if (f.type == kMix) {
+        // the other material at the sampled direction, also where sampling gave up
+        Bsdf own = f, other = f;
+        set_material(own, *f.sub[s.second ? 1 : 0]);
+        set_material(other, *f.sub[s.second ? 0 : 1]);
+        Col f_own = col(0.f, 0.f, 0.f), f_other = col(0.f, 0.f, 0.f);
+        float pdf_own = 0.f, pdf_other = 0.f;
+        if (s.ok) f_own = leaf_sampled_value(own, wo, s, pdf_own);
+        if (possible_for(other, dot(f.n, s.wi))) f_other = leaf_value(other, wo, s.wi, pdf_other);
+        const Col f1 = s.second ? f_other : f_own, f2 = s.second ? f_own : f_other;
+        const float pdf1 = s.second ? pdf_other : pdf_own, pdf2 = s.second ? pdf_own : pdf_other;
+        pdf = (1.f - f.mix_p) * pdf1 + f.mix_p * pdf2;
+        return (col(1.f, 1.f, 1.f) - f.mix_coeff) * f1 + f.mix_coeff * f2;
+    }
+    return leaf_sampled_value(f, wo, s, pdf);
 }
+// The value towards wi and the density of sampling it.
 template <bool FULL = true>
-__device__ __forceinline__ Col bsdf_evaluate(const Bsdf& f, V3 wo, V3 wi) {
-    if constexpr (FULL) return bsdf_evaluate_full(f, wo, wi);
-    else return bsdf_evaluate_body<false>(f, wo, wi);
+__device__ __forceinline__ Col bsdf_value(const Bsdf& f, V3 wo, V3 wi, float& pdf) {
+    if constexpr (FULL) return bsdf_value_full(f, wo, wi, pdf);
+    else return plain_value(f, wo, wi, false, wi, pdf);
 }
+// A sampled direction; false where the sample is black whatever its value.
 template <bool FULL = true>
-__device__ __forceinline__ float bsdf_pdf(const Bsdf& f, V3 wo, V3 wi) {
-    if constexpr (FULL) return bsdf_pdf_full(f, wo, wi);
-    else return bsdf_pdf_body<false>(f, wo, wi);
+__device__ __forceinline__ bool bsdf_direction(const Bsdf& f, float u0, float u1, float u_scatter, V3 wo,
+                                               Bsdf_Sample& s) {
+    if constexpr (FULL) s = bsdf_direction_full(f, u0, u1, u_scatter, wo);
+    else s = leaf_direction<false>(f, u0, u1, u_scatter, wo);
+    return s.ok || (FULL && f.type == kMix);
 }
+// Its value and density.
+template <bool FULL = true>
+__device__ __forceinline__ Col bsdf_sampled_value(const Bsdf& f, V3 wo, const Bsdf_Sample& s, float& pdf) {
+    if constexpr (FULL) return bsdf_sampled_value_full(f, wo, s, pdf);
+    else return plain_value(f, wo, s.wi, true, s.wh, pdf);
+}
+// BSDF::sample; black when no direction is produced.
 template <bool FULL = true>
 __device__ __forceinline__ Col bsdf_sample(const Bsdf& f, float u0, float u1, float u_scatter, V3 wo, V3& wi,
                                            float& pdf) {
-    if constexpr (FULL) return bsdf_sample_full(f, u0, u1, u_scatter, wo, wi, pdf);
-    else return bsdf_sample_plain(f, u0, u1, u_scatter, wo, wi, pdf);
+    Bsdf_Sample s;
+    const bool alive = bsdf_direction<FULL>(f, u0, u1, u_scatter, wo, s);
+    wi = s.wi;
+    return alive ? bsdf_sampled_value<FULL>(f, wo, s, pdf) : col(0.f, 0.f, 0.f);
 }
 
 // mis_power_heuristic (src/ref/direct_lighting.cpp:18-24)

@@ -1526,7 +1526,7 @@ shade_kernel(Render_Params p, Scene_Dev S, int cur, uint32_t count, const float*
                             }
                         }
                         if (lit) {
-                            const Col fv = bsdf_evaluate<FULL>(f, sc.wo, wi);
+                            const Col fv = bsdf_evaluate(f, sc.wo, wi);
                             if (kind != YAR_LIGHT_SPOT || !black(fv)) {  // only the spot light skips a black BSDF
                                 const Col c = mul(col(dc.x, dc.y, dc.z) * fv, scale);
                                 ps.pend_light[slot] = make_float4(c.r, c.g, c.b, 0.f);
@@ -1553,9 +1553,9 @@ shade_kernel(Render_Params p, Scene_Dev S, int cur, uint32_t count, const float*
                             const V3 wi = divs(lv, dist);
                             const float ndw = dot(sc.n, wi);
                             if ((ndw > 0.f && f.reflection) || (ndw < 0.f && f.transmission)) {
-                                const Col fv = bsdf_evaluate<FULL>(f, sc.wo, wi);
+                                float bpdf;
+                                const Col fv = bsdf_value<FULL>(f, sc.wo, wi, bpdf);
                                 if (!black(fv)) {
-                                    const float bpdf = bsdf_pdf<FULL>(f, sc.wo, wi);
                                     const float w = mis_power(ss.cone_pdf, bpdf);
                                     const Col c = mul(Le * fv, w * fabsf(ndw) / ss.cone_pdf);
                                     ps.pend_light[slot] = make_float4(c.r, c.g, c.b, 0.f);
@@ -1567,10 +1567,14 @@ shade_kernel(Render_Params p, Scene_Dev S, int cur, uint32_t count, const float*
                             }
                         }
                         {   // BSDF-sampling half of MIS: inside the light's cone, the probe must hit it
-                            V3 wi = v3(0.f, 0.f, 0.f);
+                            Bsdf_Sample bs;
+                            const bool alive = bsdf_direction<FULL>(f, ub.x, ub.y, u_sc, sc.wo, bs);
+                            const V3 wi = bs.wi;
                             float bpdf = 0.f;
-                            const Col fv = bsdf_sample<FULL>(f, ub.x, ub.y, u_sc, sc.wo, wi, bpdf);
-                            if (!black(fv) && dot(-ss.axes[2], wi) >= ss.cos_theta_max) {
+                            Col fv = col(0.f, 0.f, 0.f);
+                            if (alive && dot(-ss.axes[2], wi) >= ss.cos_theta_max)
+                                fv = bsdf_sampled_value<FULL>(f, sc.wo, bs, bpdf);
+                            if (!black(fv)) {
                                 const V3 position = origin_for_direction(sc, wi);
                                 const Col lef = Le * fv;
                                 ps.pend_probe0[slot] = make_float4(lef.r, lef.g, lef.b, bpdf);
@@ -1592,10 +1596,10 @@ shade_kernel(Render_Params p, Scene_Dev S, int cur, uint32_t count, const float*
                             const Col Le = env_light_sample(S, ul.x, ul.y, wi, light_pdf);
                             const float ndw = dot(sc.n, wi);
                             if ((ndw > 0.f && f.reflection) || (ndw < 0.f && f.transmission)) {
-                                const Col fv = bsdf_evaluate<FULL>(f, sc.wo, wi);
+                                float bpdf;
+                                const Col fv = bsdf_value<FULL>(f, sc.wo, wi, bpdf);
                                 if (!black(fv)) {
                                     const V3 position = origin_for_direction(sc, wi);
-                                    const float bpdf = bsdf_pdf<FULL>(f, sc.wo, wi);
                                     const float w = mis_power(light_pdf, bpdf);
                                     const Col c = mul(Le * fv, w * fabsf(ndw) / light_pdf);
                                     ps.pend_light[slot] = make_float4(c.r, c.g, c.b, 0.f);
@@ -1643,9 +1647,9 @@ shade_kernel(Render_Params p, Scene_Dev S, int cur, uint32_t count, const float*
                                 const V3 wi = divs(lv, dist);
                                 const float ndw = dot(sc.n, wi);
                                 if ((ndw > 0.f && f.reflection) || (ndw < 0.f && f.transmission)) {
-                                    const Col fv = bsdf_evaluate<FULL>(f, sc.wo, wi);
+                                    float bpdf;
+                                    const Col fv = bsdf_value<FULL>(f, sc.wo, wi, bpdf);
                                     if (!black(fv)) {
-                                        const float bpdf = bsdf_pdf<FULL>(f, sc.wo, wi);
                                         const float w = mis_power(light_pdf, bpdf);
                                         const Col c = mul(Le * fv, w * fabsf(ndw) / light_pdf);
                                         ps.pend_light[slot] = make_float4(c.r, c.g, c.b, 0.f);
@@ -1694,10 +1698,10 @@ shade_kernel(Render_Params p, Scene_Dev S, int cur, uint32_t count, const float*
                                 const float ndw = dot(sc.n, wi);
                                 const bool possible = (ndw > 0.f && f.reflection) || (ndw < 0.f && f.transmission);
                                 if (possible) {
-                                    const Col fv = bsdf_evaluate<FULL>(f, sc.wo, wi);
+                                    float bpdf;
+                                    const Col fv = bsdf_value<FULL>(f, sc.wo, wi, bpdf);
                                     if (!black(fv)) {
                                         const float light_pdf = (dist * dist) / (size_x * size_y * lndw);
-                                        const float bpdf = bsdf_pdf<FULL>(f, sc.wo, wi);
                                         const float w = mis_power(light_pdf, bpdf);
                                         const Col c = mul(Le * fv, w * fabsf(ndw) / light_pdf);
                                         ps.pend_light[slot] = make_float4(c.r, c.g, c.b, 0.f);
@@ -1710,13 +1714,16 @@ shade_kernel(Render_Params p, Scene_Dev S, int cur, uint32_t count, const float*
                             }
                         }
                         {   // BSDF-sampling half of MIS: the probe ray must hit this light
-                            V3 wi = v3(0.f, 0.f, 0.f);
-                            float bpdf = 0.f;
-                            const Col fv = bsdf_sample<FULL>(f, ub.x, ub.y, u_sc, sc.wo, wi, bpdf);
-                            if (!black(fv)) {
+                            Bsdf_Sample bs;
+                            if (bsdf_direction<FULL>(f, ub.x, ub.y, u_sc, sc.wo, bs)) {
+                                const V3 wi = bs.wi;
                                 const float lndw = dot(light_n, -wi);
                                 const V3 position = origin_for_direction(sc, wi);
-                                if (lndw > 1e-4f && probe_may_reach(Ld, position, wi, lndw)) {
+                                float bpdf = 0.f;
+                                Col fv = col(0.f, 0.f, 0.f);
+                                if (lndw > 1e-4f && probe_may_reach(Ld, position, wi, lndw))
+                                    fv = bsdf_sampled_value<FULL>(f, sc.wo, bs, bpdf);
+                                if (!black(fv)) {
                                     const Col lef = Le * fv;
                                     ps.pend_probe0[slot] = make_float4(lef.r, lef.g, lef.b, bpdf);
                                     ps.pend_probe1[slot] = make_float4(position.x, position.y, position.z, lndw);
@@ -1774,8 +1781,7 @@ shade_kernel(Render_Params p, Scene_Dev S, int cur, uint32_t count, const float*
                                 wi = mixture_sample(lob, u_scatter_next, un.x, un.y);
                                 const float ndw = dot(sc.n, wi);
                                 const bool possible = (ndw > 0.f && f.reflection) || (ndw < 0.f && f.transmission);
-                                fv = possible ? bsdf_evaluate<FULL>(f, sc.wo, wi) : col(0.f, 0.f, 0.f);
-                                pdf_b = possible ? bsdf_pdf<FULL>(f, sc.wo, wi) : 0.f;
+                                fv = possible ? bsdf_value<FULL>(f, sc.wo, wi, pdf_b) : col(0.f, 0.f, 0.f);
                             } else {
                                 fv = bsdf_sample<FULL>(f, un.x, un.y, u_scatter_next, sc.wo, wi, pdf_b);
                             }
