@@ -130,7 +130,7 @@ struct Render_Params {
     float filter_zero;      // gaussian: exp(-alpha r^2), the weight at the radius (computed on the host)
     float film_scale, max_component;
     int32_t total_lights, delta_lights, rect_lights, sphere_lights, mesh_lights, env_lights;  // selection order
-    int32_t full_shading;  // the scene needs shade_kernel<*, true>
+    int32_t full_shading;  // the scene needs more than shade_kernel<*, kShadePlain>
     int32_t arrays_2d_first;  // direct lighting: the 2D rows (array grids) come before the 1D rows in the stream
     uint32_t seed_offset;
     uint32_t stream_hi;  // upper 32 bits of the pixel streams' sequence (0 = the reference's streams)
@@ -1328,26 +1328,31 @@ __device__ __forceinline__ V3 sphere_sampler_sample(const Sphere_Sampler& ss, fl
 // alpha q + (1 - alpha) p_bsdf, so the estimator stays unbiased; the light
 // sample and the MIS probe are unchanged.  With g.records set, every
 // continued vertex also leaves a training record.
-// FULL: delta materials, the layered, translucent and mixed BSDFs, and every
-// light kind but the quad light.  A scene without them runs the FULL = false
-// instantiation, which has none of that code (launch_shade picks it from
-// Render_Params::full_shading).
-// Launch bounds: the plain instantiation (diffuse, metal, rough glass, quad
-// lights: the C1, C3 and batch renders) at 4 blocks of 128 threads per SM
-// (128 registers) spills nothing: the shadow, probe and next extend rays wait
-// for the warp's appends in shared memory, and the path's radiance is read and
-// written only where emission adds to it; its guided form spills 18 B.  The
-// FULL instantiations keep 3 blocks (160-162 registers, no spills; at 4 the
-// out-of-line BSDF routines, the fourier series among them, push the kernel
-// to 36-60 B of spills).  The guided plain-material form at 3 blocks (152
-// registers, no spills) rendered the guided room no faster than at 4 (38 B
-// of spills).  Before those changes the plain kernel ran at 5
-// blocks (96 registers, 202 B of spill stores), which measured 1.726 s on the
-// C3 render against 1.732 s at 4 blocks and 1.764 s at 3.
-template <bool GUIDED, bool FULL>
-__global__ void __launch_bounds__(kBlock, FULL ? 3 : 4)
+// KIND (launch_shade picks it from Render_Params): kShadePlain for diffuse,
+// metal and rough glass under quad lights, kShadeFull with delta materials,
+// the layered, translucent and mixed BSDFs and every other light kind,
+// kShadeTextured with image textures and bump maps on top.
+// Bounds: the plain kernel waits on its own arithmetic (divisions and square
+// roots, 3,000 instructions per vertex at 43% of the issue slots) and on
+// loads; at 4 blocks of 128 threads per SM it spills nothing, with the
+// shadow, probe and next extend rays waiting for the warp's appends in shared
+// memory and the path's radiance read and written only where emission adds to
+// it.  The GGX room, 512 x 512 samples of 64: 39.7 ms at 4 blocks, 41.7 at 3,
+// 40.5 at 5, 39.9 at 6; its guided form spills 18 B.  kShadeFull at 3 blocks
+// (164 registers, no spills): 6.54 ms for the box with point, spot and
+// distant lights, 6.91 at 4, 7.11 at 2.  kShadeTextured walks mip levels, one
+// dependent load after another, so resident warps count more than spills: the
+// bump-mapped box took 38.9 ms at 4 blocks, 36.2 at 5, 32.5 at 8 (1.4 KB of
+// spills); delta materials with textures 28.2, 27.8 and 26.2 ms, a small image
+// of them (333 x 250) 5.40, 5.42 and 5.49 ms.  With the texture code in
+// kShadeFull at 3 blocks: 39.2, 28.4 and 5.56 ms, and 6.91 ms for the lights.
+enum Shade_Kind { kShadePlain, kShadeFull, kShadeTextured };
+constexpr int kShadeBlocks[3] = {4, 3, 8};
+template <bool GUIDED, int KIND>
+__global__ void __launch_bounds__(kBlock, kShadeBlocks[KIND])
 shade_kernel(Render_Params p, Scene_Dev S, int cur, uint32_t count, const float* __restrict__ s1d,
              const float2* __restrict__ s2d, Path_State ps, Queues q, Guide_Shade g) {
+    constexpr bool FULL = KIND != kShadePlain, TEXTURED = KIND == kShadeTextured;
     // this thread's shadow, probe and next extend rays (origin + tmax,
     // direction) from where they are made until the warp's appends: in shared
     // memory, not in 24 registers live across the whole shading
@@ -1453,7 +1458,7 @@ shade_kernel(Render_Params p, Scene_Dev S, int cur, uint32_t count, const float*
                 // src/ref/delta_scattering.cpp:252-257; create_bsdf again, which
                 // gives the same frame).
                 Tex_Site site;
-                const bool textured = FULL && (mat.texture | mat.texture2 | mat.bump) != 0u;
+                const bool textured = TEXTURED && (mat.texture | mat.texture2 | mat.bump) != 0u;
                 if (textured) {
                     texture_site(p, S, ps, slot, bounce, info, sc, h4, h2, site);
                     if (mat.bump) apply_bump(S, mat, site, h2.y, h2.x, h4.y, h4.z, h4.w, sc);
@@ -1745,7 +1750,7 @@ shade_kernel(Render_Params p, Scene_Dev S, int cur, uint32_t count, const float*
                     // Reflected and transmitted delta rays carry differential rays for
                     // the first max_differential_ray_specular_bounces bounces.
                     uint32_t diff_flag = 0u;
-                    if (FULL && p.spec_diffs && delta == 1 && delta_kind >= 0.f &&
+                    if (TEXTURED && p.spec_diffs && delta == 1 && delta_kind >= 0.f &&
                         bounce < kMaxDifferentialRaySpecularBounces &&
                         specular_differentials(p, S, ps, slot, bounce, info, sc, h4, h2, delta_wi, delta_kind))
                         diff_flag = kDiffRays;
@@ -1877,10 +1882,10 @@ shade_kernel(Render_Params p, Scene_Dev S, int cur, uint32_t count, const float*
 template <bool GUIDED>
 void launch_shade(const Render_Params& p, unsigned grid, cudaStream_t st, const Scene_Dev& S, int cur, uint32_t count,
                   const float* s1d, const float2* s2d, const Path_State& ps, const Queues& q, const Guide_Shade& g) {
-    if (p.full_shading)
-        shade_kernel<GUIDED, true><<<grid, kBlock, 0, st>>>(p, S, cur, count, s1d, s2d, ps, q, g);
-    else
-        shade_kernel<GUIDED, false><<<grid, kBlock, 0, st>>>(p, S, cur, count, s1d, s2d, ps, q, g);
+    auto kernel = p.textured       ? shade_kernel<GUIDED, kShadeTextured>
+                  : p.full_shading ? shade_kernel<GUIDED, kShadeFull>
+                                   : shade_kernel<GUIDED, kShadePlain>;
+    kernel<<<grid, kBlock, 0, st>>>(p, S, cur, count, s1d, s2d, ps, q, g);
 }
 
 // ---------------------------------------------------------------- connect
