@@ -232,8 +232,8 @@ cudaError_t enqueue_scene(Batch& bt, int si, bool one_spp, unsigned long long* s
             if (mixed) {
                 uint32_t* bins = dp<uint32_t>(br.B[29]);
                 cudaMemsetAsync(bins, 0, 2 * kShadeClasses * sizeof(uint32_t), st);
-                shade_bin_kernel<<<kFixedGrid, kBlock, 0, st>>>(S, q, paths, dp<uint8_t>(br.B[27]), bins);
-                shade_order_kernel<<<kFixedGrid, kBlock, 0, st>>>(q, paths, dp<uint8_t>(br.B[27]), bins,
+                shade_bin_kernel<<<kShadeOrderBlocks, kBlock, 0, st>>>(S, q, paths, dp<uint8_t>(br.B[27]), bins);
+                shade_order_kernel<<<kShadeOrderBlocks, kBlock, 0, st>>>(q, paths, dp<uint8_t>(br.B[27]), bins,
                                                                   dp<uint32_t>(br.B[28]));
             }
             launch_shade<false>(p, kFixedGrid, st, S, cur, paths, dp<float>(br.B[2]), dp<float2>(br.B[3]), ps, qs,

@@ -622,8 +622,8 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
     auto order_queue = [&](const Queues& qq, uint32_t max_count, int grid) {
         if (!mixed) return;
         cudaMemsetAsync(shade_bins, 0, 2 * kShadeClasses * sizeof(uint32_t), st);
-        shade_bin_kernel<<<grid, kBlock, 0, st>>>(S, qq, max_count, shade_keys, shade_bins);
-        shade_order_kernel<<<grid, kBlock, 0, st>>>(qq, max_count, shade_keys, shade_bins,
+        shade_bin_kernel<<<std::min(grid, kShadeOrderBlocks), kBlock, 0, st>>>(S, qq, max_count, shade_keys, shade_bins);
+        shade_order_kernel<<<std::min(grid, kShadeOrderBlocks), kBlock, 0, st>>>(qq, max_count, shade_keys, shade_bins,
                                                     const_cast<uint32_t*>(qo.order));
     };
     // The rays of bounces after the camera's, sorted by direction octant and

@@ -1992,43 +1992,81 @@ __device__ __forceinline__ void key_group(uint32_t key, uint32_t& rank, int& lea
     size = __popc(group);
 }
 
+// Both kernels below are bound by the queue's bytes (9 and 5 B per entry) once
+// their atomics on the few class counters are few: one per class and block
+// here, one per class and kOrderItems entries there.  Over a render of 2.4M
+// triangles at 1080p (76 bounces of two chunks) they took 2.0 ms each with one
+// atomic per class and warp (a million on four words for the first bounce),
+// 0.44 and 0.60 ms as below.
+constexpr int kShadeOrderBlocks = 152 * 16;
+
 // bins[0..3]: the queue's entries per class (bins zeroed by the caller).
 __global__ void __launch_bounds__(kBlock)
 shade_bin_kernel(Scene_Dev S, Queues q, uint32_t count, uint8_t* __restrict__ keys, uint32_t* __restrict__ bins) {
     if (q.ext_count) count = *q.ext_count;
+    __shared__ uint32_t total[kShadeClasses];
+    if (threadIdx.x < kShadeClasses) total[threadIdx.x] = 0u;
+    __syncthreads();
+    uint32_t n[kShadeClasses] = {};  // of this warp
     for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += gridDim.x * blockDim.x) {
         const uint32_t i = base + threadIdx.x;
         const uint32_t key = i < count ? shade_class(S, q.ext_hit2[i]) : kShadeClasses;
         if (i < count) keys[i] = (uint8_t)key;
-        uint32_t rank, size;
-        int leader;
-        key_group(key, rank, leader, size);
-        if (i < count && rank == 0) atomicAdd(&bins[key], size);
+#pragma unroll
+        for (uint32_t c = 0; c < kShadeClasses; c++) n[c] += __popc(__ballot_sync(0xffffffffu, key == c));
     }
+    if ((threadIdx.x & 31u) == 0u)
+        for (uint32_t c = 0; c < kShadeClasses; c++) atomicAdd(&total[c], n[c]);
+    __syncthreads();
+    if (threadIdx.x < kShadeClasses && total[threadIdx.x]) atomicAdd(&bins[threadIdx.x], total[threadIdx.x]);
 }
 
 // order[]: the queue's entries class after class (bins[4..7] hand out the
 // places within a class).
+constexpr uint32_t kOrderRounds = 8, kOrderItems = kOrderRounds * kBlock;  // entries a block places at a time
 __global__ void __launch_bounds__(kBlock)
 shade_order_kernel(Queues q, uint32_t count, const uint8_t* __restrict__ keys, uint32_t* __restrict__ bins,
                    uint32_t* __restrict__ order) {
     if (q.ext_count) count = *q.ext_count;
-    uint32_t first[kShadeClasses];
-    uint32_t acc = 0;
-    for (uint32_t c = 0; c < kShadeClasses; c++) {
-        first[c] = acc;
-        acc += bins[c];
-    }
-    for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += gridDim.x * blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        const uint32_t key = i < count ? keys[i] : kShadeClasses;
-        uint32_t rank, size;
-        int leader;
-        key_group(key, rank, leader, size);
-        uint32_t at = 0;
-        if (i < count && rank == 0) at = atomicAdd(&bins[kShadeClasses + key], size);
-        at = __shfl_sync(0xffffffffu, at, leader);
-        if (i < count) order[first[key] + at + rank] = i;
+    __shared__ uint32_t place[kBlock / 32][kShadeClasses];  // a warp's counts, then its first places
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, lower = (1u << lane) - 1u;
+    uint32_t first = 0;  // of class threadIdx.x
+    for (uint32_t c = 0; c < kShadeClasses && c < threadIdx.x; c++) first += bins[c];
+    for (uint32_t base = blockIdx.x * kOrderItems; base < count; base += gridDim.x * kOrderItems) {
+        const uint32_t i0 = base + warp * (32u * kOrderRounds) + lane;
+        uint32_t key[kOrderRounds], n[kShadeClasses] = {};
+#pragma unroll
+        for (uint32_t r = 0; r < kOrderRounds; r++) key[r] = i0 + 32u * r < count ? keys[i0 + 32u * r] : kShadeClasses;
+#pragma unroll
+        for (uint32_t r = 0; r < kOrderRounds; r++)
+#pragma unroll
+            for (uint32_t c = 0; c < kShadeClasses; c++) n[c] += __popc(__ballot_sync(0xffffffffu, key[r] == c));
+        if (lane == 0)
+#pragma unroll
+            for (uint32_t c = 0; c < kShadeClasses; c++) place[warp][c] = n[c];
+        __syncthreads();
+        if (threadIdx.x < kShadeClasses) {
+            uint32_t sum = 0;
+            for (uint32_t w = 0; w < kBlock / 32; w++) sum += place[w][threadIdx.x];
+            uint32_t at = first + (sum ? atomicAdd(&bins[kShadeClasses + threadIdx.x], sum) : 0u);
+            for (uint32_t w = 0; w < kBlock / 32; w++) {
+                const uint32_t size = place[w][threadIdx.x];
+                place[w][threadIdx.x] = at;
+                at += size;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (uint32_t c = 0; c < kShadeClasses; c++) n[c] = place[warp][c];
+#pragma unroll
+        for (uint32_t r = 0; r < kOrderRounds; r++)
+#pragma unroll
+            for (uint32_t c = 0; c < kShadeClasses; c++) {
+                const unsigned mask = __ballot_sync(0xffffffffu, key[r] == c);
+                if (key[r] == c) order[n[c] + __popc(mask & lower)] = i0 + 32u * r;
+                n[c] += __popc(mask);
+            }
+        __syncthreads();  // `place` is written again
     }
 }
 
