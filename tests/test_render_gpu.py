@@ -305,6 +305,27 @@ def test_render_direct_lighting_split_over_launches(gpu_ctx, scene, width, heigh
     assert stats.variance == ref_var
 
 
+@pytest.mark.parametrize("region", [(0, 0, 65, 63), (16350, 16320, 16383, 16385)])
+@pytest.mark.parametrize("nx,ny", [(1, 1), (2, 1), (3, 1), (2, 2), (5, 1), (3, 3), (4, 4), (17, 1)])
+def test_film_sums_of_every_sample_count(gpu_ctx, region, nx, ny):
+    """Sample counts around the widths the film's sums are taken in, tile and
+    warp edges, and pixels so far out that rounding moves samples onto the next
+    one: as the oracle."""
+    s = FlatScene.read(golden("cornell_c1_64.yfs"))
+    s.camera, s.config = np.array(s.camera), np.array(s.config)
+    extent = (max(64, region[2]), max(64, region[3]))
+    s.camera["image_extent"] = extent
+    s.camera["horz_half_dist"] = np.float32(np.float32(extent[0]) / np.float32(extent[1])) * s.camera["vert_half_dist"]
+    s.config["render_region"] = region
+    s.config["x_pixel_sample_count"], s.config["y_pixel_sample_count"] = nx, ny
+    s.config["max_light_bounces"] = 2
+    ref, ref_var = oracle.render(s, threads=8, correctly_rounded_trig=True)
+    gpu_ctx.upload_scene(s)
+    img, stats = gpu_ctx.render(region[2] - region[0], region[3] - region[1])
+    assert np.array_equal(img.view(np.uint32), ref.view(np.uint32))
+    assert stats.variance == ref_var
+
+
 def test_render_unsupported_features_fail_cleanly(gpu_ctx):
     from yar_gb300 import native
     s = FlatScene.read(golden("cornell_c1_64.yfs"))

@@ -271,13 +271,12 @@ cudaError_t enqueue_scene(Batch& bt, int si, bool one_spp, unsigned long long* s
         if (e == cudaSuccess) e = cudaGetLastError();
     }
     if (e != cudaSuccess) return e;
-    samples_kernel<<<(uint32_t)((sc.pixels + kBlock - 1) / kBlock), kBlock, 0, st>>>(p, dp<float4>(sc.radiance),
-                                                                                   dp<double>(sc.pixel_var));
-    tile_variance_kernel<<<p.tiles_x * p.tiles_y, kTileVarThreads, 0, st>>>(p, dp<double>(sc.pixel_var),
-                                                                            dp<double>(sc.tile_var));
+    const Pixel_Film pf = pixel_film(p, sc.pixel_var.ptr, sc.pixels);
+    launch_samples(p, dp<float4>(sc.radiance), dp<float2>(sc.image_samples), pf, st);
+    tile_variance_kernel<<<p.tiles_x * p.tiles_y, kTileVarThreads, 0, st>>>(p, pf.variance, dp<double>(sc.tile_var));
     variance_total_kernel<<<1, 1, 0, st>>>(p, dp<double>(sc.tile_var), dp<double>(sc.variance));
     film_kernel<<<(uint32_t)(((uint64_t)p.rw * p.rh + kBlock - 1) / kBlock), kBlock, 0, st>>>(
-        p, dp<float4>(sc.radiance), dp<float2>(sc.image_samples), dp<float>(sc.rgb));
+        p, dp<float4>(sc.radiance), dp<float2>(sc.image_samples), pf, dp<float>(sc.rgb));
     stamp_kernel<<<1, 1, 0, st>>>(stamp);
     return cudaGetLastError();
 }
@@ -371,7 +370,7 @@ int render_batch(yar_gpu_ctx* ctx, const yar_flat_scene* const* scenes, uint32_t
         if (s.samples > 0xffffffffull) return fail(ctx, YAR_ERR_CAPACITY, "render batch: too many samples in a scene");
         if ((rc = device_alloc(ctx, s.radiance, s.samples * sizeof(float4))) != YAR_OK) return rc;
         if ((rc = device_alloc(ctx, s.image_samples, s.samples * sizeof(float2))) != YAR_OK) return rc;
-        if ((rc = device_alloc(ctx, s.pixel_var, s.pixels * sizeof(double))) != YAR_OK) return rc;
+        if ((rc = device_alloc(ctx, s.pixel_var, pixel_film_bytes(s.pixels))) != YAR_OK) return rc;
         if ((rc = device_alloc(ctx, s.tile_var, (size_t)s.p.tiles_x * s.p.tiles_y * sizeof(double))) != YAR_OK)
             return rc;
         if ((rc = device_alloc(ctx, s.variance, sizeof(double))) != YAR_OK) return rc;

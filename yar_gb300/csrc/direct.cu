@@ -677,7 +677,7 @@ int render_direct(yar_gpu_ctx* ctx, float* rgb_out, yar_render_stats* stats) {
         alloc(11, cap * sizeof(float4));                      // hit4 of camera and delta rays
         alloc(12, cap * sizeof(uint2));                       // hit2
         alloc(13, cap * sizeof(uint32_t));                    // draw offsets
-        alloc(14, pixels * sizeof(double));                   // pixel variance
+        alloc(14, pixel_film_bytes(pixels));                  // pixel variance, film sums
         alloc(15, (size_t)p.tiles_x * p.tiles_y * sizeof(double));
         alloc(16, (size_t)p.rw * p.rh * 3 * sizeof(float));   // rgb
         alloc(17, 2 * sizeof(unsigned long long) + 4 * sizeof(int));  // ray counts, traversal error
@@ -809,12 +809,11 @@ int render_direct(yar_gpu_ctx* ctx, float* rgb_out, yar_render_stats* stats) {
         if (e == cudaSuccess) e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
-        samples_kernel<<<(uint32_t)((pixels + kBlock - 1) / kBlock), kBlock, 0, st>>>(p, dptr<float4>(B[0]),
-                                                                                      dptr<double>(B[14]));
-        tile_variance_kernel<<<p.tiles_x * p.tiles_y, kTileVarThreads, 0, st>>>(p, dptr<double>(B[14]),
-                                                                                dptr<double>(B[15]));
+        const Pixel_Film pf = pixel_film(p, B[14].ptr, pixels);
+        launch_samples(p, dptr<float4>(B[0]), dptr<float2>(B[1]), pf, st);
+        tile_variance_kernel<<<p.tiles_x * p.tiles_y, kTileVarThreads, 0, st>>>(p, pf.variance, dptr<double>(B[15]));
         film_kernel<<<(uint32_t)(((uint64_t)p.rw * p.rh + kBlock - 1) / kBlock), kBlock, 0, st>>>(
-            p, dptr<float4>(B[0]), dptr<float2>(B[1]), dptr<float>(B[16]));
+            p, dptr<float4>(B[0]), dptr<float2>(B[1]), pf, dptr<float>(B[16]));
         launches += 3;
         e = cudaGetLastError();
     }

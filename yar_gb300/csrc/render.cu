@@ -545,7 +545,7 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
     alloc(24, cap * 2 * sizeof(float4));                   // probe rays
     alloc(25, cap * sizeof(uint32_t));                     // probe slots
     alloc(26, 8 * sizeof(uint32_t));                       // counters
-    alloc(27, pixels * sizeof(double));                    // pixel variance
+    alloc(27, pixel_film_bytes(pixels));                   // pixel variance, film sums
     alloc(28, (size_t)p.tiles_x * p.tiles_y * sizeof(double));
     alloc(29, (size_t)p.rw * p.rh * 3 * sizeof(float));    // rgb
     if (p.exact_tail) {
@@ -811,7 +811,8 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
         launches++;
     }
     if (e == cudaSuccess) {
-        samples_kernel<<<(uint32_t)((pixels + kBlock - 1) / kBlock), kBlock, 0, st>>>(p, radiance, dptr<double>(B[27]));
+        const Pixel_Film pf = pixel_film(p, B[27].ptr, pixels);
+        launch_samples(p, radiance, image_samples, pf, st);
         // the tile sums (one sequential FP64 chain per 64 x 64 tile, the
         // reference's order) run on a second stream beside the film
         if (!ctx->aux_stream) e = cudaStreamCreateWithFlags(&ctx->aux_stream, cudaStreamNonBlocking);
@@ -821,11 +822,11 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
         if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->aux_stream, ctx->aux_fork, 0);
         if (e == cudaSuccess)
             tile_variance_kernel<<<p.tiles_x * p.tiles_y, kTileVarThreads, 0, ctx->aux_stream>>>(
-                p, dptr<double>(B[27]), dptr<double>(B[28]));
+                p, pf.variance, dptr<double>(B[28]));
         launches += 2;
         if (e == cudaSuccess && !tiles_out) {
             film_kernel<<<(uint32_t)(((uint64_t)p.rw * p.rh + kBlock - 1) / kBlock), kBlock, 0, st>>>(
-                p, radiance, image_samples, dptr<float>(B[29]));
+                p, radiance, image_samples, pf, dptr<float>(B[29]));
             launches++;
         }
         if (e == cudaSuccess) e = cudaEventRecord(ctx->aux_join, ctx->aux_stream);
@@ -1102,11 +1103,12 @@ int render_run_static(yar_gpu_ctx* ctx, float* rgb_out_device, yar_render_stats*
     }
     double variance = 0.0;
     if (e == cudaSuccess) {
-        samples_kernel<<<(uint32_t)((pixels + kBlock - 1) / kBlock), kBlock, 0, st>>>(p, radiance, pixel_variance);
+        const Pixel_Film pf{pixel_variance, nullptr, nullptr};  // (the arena holds no film sums)
+        launch_samples(p, radiance, image_samples, pf, st);
         tile_variance_kernel<<<(uint32_t)tiles, kTileVarThreads, 0, st>>>(p, pixel_variance, tile_variance);
         variance_total_kernel<<<1, 1, 0, st>>>(p, tile_variance, variance_total);
         film_kernel<<<(uint32_t)(((uint64_t)p.rw * p.rh + kBlock - 1) / kBlock), kBlock, 0, st>>>(
-            p, radiance, image_samples, rgb_out_device);
+            p, radiance, image_samples, pf, rgb_out_device);
         launches += 4;
         e = cudaGetLastError();
     }
