@@ -1338,7 +1338,9 @@ __device__ __forceinline__ V3 sphere_sampler_sample(const Sphere_Sampler& ss, fl
 // shadow, probe and next extend rays waiting for the warp's appends in shared
 // memory and the path's radiance read and written only where emission adds to
 // it.  The GGX room, 512 x 512 samples of 64: 39.7 ms at 4 blocks, 41.7 at 3,
-// 40.5 at 5, 39.9 at 6; its guided form spills 18 B.  kShadeFull at 3 blocks
+// 40.5 at 5, 39.9 at 6; its guided form, which also waits on the mixtures it
+// reads, renders that room in 38.3 ms at 4, 40.3 at 3, 38.1 at 5, 37.6 at 6
+// and 38.0 at 8.  kShadeFull at 3 blocks
 // (164 registers, no spills): 6.54 ms for the box with point, spot and
 // distant lights, 6.91 at 4, 7.11 at 2.  kShadeTextured walks mip levels, one
 // dependent load after another, so resident warps count more than spills: the
@@ -1349,7 +1351,7 @@ __device__ __forceinline__ V3 sphere_sampler_sample(const Sphere_Sampler& ss, fl
 enum Shade_Kind { kShadePlain, kShadeFull, kShadeTextured };
 constexpr int kShadeBlocks[3] = {4, 3, 8};
 template <bool GUIDED, int KIND>
-__global__ void __launch_bounds__(kBlock, kShadeBlocks[KIND])
+__global__ void __launch_bounds__(kBlock, GUIDED && KIND == kShadePlain ? 6 : kShadeBlocks[KIND])
 shade_kernel(Render_Params p, Scene_Dev S, int cur, uint32_t count, const float* __restrict__ s1d,
              const float2* __restrict__ s2d, Path_State ps, Queues q, Guide_Shade g) {
     constexpr bool FULL = KIND != kShadePlain, TEXTURED = KIND == kShadeTextured;
