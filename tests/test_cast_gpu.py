@@ -316,3 +316,31 @@ def test_alpha_test_matches_oracle(kernel):
         assert not np.array_equal(ctx.cast_any(shadow), occ)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("n", [1, 31, 8191, 8192, 8193])
+def test_small_host_casts_match_device_casts(n):
+    """Host-buffer casts on either side of the size whose results the kernels
+    write to the host themselves, with every and with one result array."""
+    torch = pytest.importorskip("torch")
+    s = scenes.raycast_scene(seed=2, grid=48, spheres=5, level=2)
+    lo, hi = scenes.scene_box(s)
+    rays = scenes.random_rays(lo, hi, n, 40 + n, tmax=np.inf)
+    shadow = scenes.random_rays(lo, hi, n, 50 + n, tmax=3.0)
+    ctx = native.Context(0)
+    ctx.upload_scene(s)
+    got = ctx.cast_closest(rays) + (ctx.cast_any(shadow),)
+    alone = np.zeros(n, np.uint32)  # the object only
+    hits = native.HitSoa(None, None, native._ptr(alone), None)
+    assert native.lib().yar_gpu_cast_closest(ctx._h, native._ptr(rays), n, native.C.byref(hits),
+                                             native.YAR_BUFFERS_HOST) == 0
+    out = [torch.zeros(n, dtype=torch.int32, device="cuda") for _ in range(3)]
+    out += [torch.zeros((n, 2), dtype=torch.float32, device="cuda"), torch.zeros(n, dtype=torch.uint8, device="cuda")]
+    dr, ds = torch.as_tensor(rays).cuda(), torch.as_tensor(shadow).cuda()
+    torch.cuda.synchronize()
+    ctx.cast_closest_device(dr.data_ptr(), n, *[o.data_ptr() for o in out[:4]])
+    ctx.cast_any_device(ds.data_ptr(), n, out[4].data_ptr())
+    for g, w in zip(got, out):
+        assert g.tobytes() == w.cpu().numpy().tobytes()
+    assert np.array_equal(alone, got[2])
+    ctx.close()

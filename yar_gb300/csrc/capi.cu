@@ -42,6 +42,17 @@ int device_alloc(yar_gpu_ctx* ctx, Device_Buffer& b, size_t bytes) {
     return YAR_OK;
 }
 
+char* pinned_block(yar_gpu_ctx* ctx) {
+    if (!ctx->pinned) {
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, kPinnedHead + (size_t)kSmallCastRays * 52, cudaHostAllocDefault) != cudaSuccess)
+            cudaGetLastError();
+        else
+            ctx->pinned = (char*)p;
+    }
+    return ctx->pinned;
+}
+
 void device_free(Device_Buffer& b) {
     if (b.ptr) cudaFree(b.ptr);
     b.ptr = nullptr;
@@ -170,6 +181,7 @@ extern "C" void yar_gpu_destroy(yar_gpu_ctx* ctx) {
     for (Device_Buffer* b : {&ctx->scene_nodes, &ctx->mesh_nodes, &ctx->objects, &ctx->tris, &ctx->d_rays, &ctx->d_t,
                              &ctx->d_prim, &ctx->d_obj, &ctx->d_bary, &ctx->d_occ, &ctx->d_answers})
         device_free(*b);
+    if (ctx->pinned) cudaFreeHost(ctx->pinned);
     if (ctx->d_error) cudaFree(ctx->d_error);
     if (ctx->d_counter) cudaFree(ctx->d_counter);
     if (ctx->ev_start) cudaEventDestroy(ctx->ev_start);
@@ -358,10 +370,12 @@ int ensure_staging(yar_gpu_ctx* ctx, uint32_t n, bool closest) {
 
 int check_error_word(yar_gpu_ctx* ctx) {
     int h = 0;
-    cudaError_t e = cudaMemcpyAsync(&h, ctx->d_error, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
+    int* word = reinterpret_cast<int*>(pinned_block(ctx));
+    if (!word) word = &h;
+    cudaError_t e = cudaMemcpyAsync(word, ctx->d_error, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "kernel");
-    if (h) {
+    if (*word) {
         cudaMemsetAsync(ctx->d_error, 0, sizeof(int), ctx->stream);
         return fail(ctx, YAR_ERR_CAPACITY, "kd-tree traversal stack overflow");
     }
@@ -493,6 +507,7 @@ int cast(yar_gpu_ctx* ctx, const yar_ray* rays, uint32_t n, const yar_hit_soa* h
     uint32_t *d_prim = nullptr, *d_obj = nullptr;
     float2* d_bary = nullptr;
     uint8_t* d_occ = nullptr;
+    char* small = buffers == YAR_BUFFERS_HOST && n <= kSmallCastRays ? pinned_block(ctx) : nullptr;
     if (buffers == YAR_BUFFERS_HOST) {
         int rc = ensure_staging(ctx, n, closest);
         if (rc != YAR_OK) return rc;
@@ -500,10 +515,22 @@ int cast(yar_gpu_ctx* ctx, const yar_ray* rays, uint32_t n, const yar_hit_soa* h
         const int tuned = wide_or_fixed;
         if (!kernel_ms && pipeline_chunks(ctx, n) >= 2 && (tuned >= 0 || n < kTuneMinRays))
             return cast_pipelined(ctx, rays, n, hits, occluded, tuned < 0 ? kCastPersistent64 : tuned);
-        e = cudaMemcpyAsync(ctx->d_rays.ptr, rays, (size_t)n * 32, cudaMemcpyHostToDevice, ctx->stream);
+        if (small) memcpy(small + kPinnedHead, rays, (size_t)n * 32);
+        e = cudaMemcpyAsync(ctx->d_rays.ptr, small ? (const void*)(small + kPinnedHead) : rays, (size_t)n * 32,
+                            cudaMemcpyHostToDevice, ctx->stream);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "ray upload");
         d_rays = (const float4*)ctx->d_rays.ptr;
-        if (closest) {
+        if (small) {  // the results straight into the block: bary, t, prim, object, or occluded
+            char* out = small + kPinnedHead + (size_t)n * 32;
+            if (closest) {
+                d_bary = hits->bary ? (float2*)out : nullptr;
+                d_t = hits->t ? (float*)(out + (size_t)n * 8) : nullptr;
+                d_prim = hits->prim ? (uint32_t*)(out + (size_t)n * 12) : nullptr;
+                d_obj = hits->object ? (uint32_t*)(out + (size_t)n * 16) : nullptr;
+            } else {
+                d_occ = (uint8_t*)out;
+            }
+        } else if (closest) {
             d_t = hits->t ? (float*)ctx->d_t.ptr : nullptr;
             d_prim = hits->prim ? (uint32_t*)ctx->d_prim.ptr : nullptr;
             d_obj = hits->object ? (uint32_t*)ctx->d_obj.ptr : nullptr;
@@ -545,7 +572,7 @@ int cast(yar_gpu_ctx* ctx, const yar_ray* rays, uint32_t n, const yar_hit_soa* h
     e = closest ? launch_extend(ctx->ds, a, k, ctx->stream) : launch_shadow(ctx->ds, a, k, ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, closest ? "extend launch" : "shadow launch");
     if (kernel_ms) cudaEventRecord(ctx->ev_stop, ctx->stream);
-    if (buffers == YAR_BUFFERS_HOST) {
+    if (buffers == YAR_BUFFERS_HOST && !small) {
         if (closest) {
             if (hits->t) e = cudaMemcpyAsync(hits->t, d_t, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream);
             if (e == cudaSuccess && hits->prim)
@@ -560,6 +587,13 @@ int cast(yar_gpu_ctx* ctx, const yar_ray* rays, uint32_t n, const yar_hit_soa* h
         if (e != cudaSuccess) return cuda_fail(ctx, e, "result download");
     }
     int rc = check_error_word(ctx);
+    if (small && rc != YAR_ERR_CUDA) {
+        if (d_t) memcpy(hits->t, d_t, (size_t)n * 4);
+        if (d_prim) memcpy(hits->prim, d_prim, (size_t)n * 4);
+        if (d_obj) memcpy(hits->object, d_obj, (size_t)n * 4);
+        if (d_bary) memcpy(hits->bary, d_bary, (size_t)n * 8);
+        if (d_occ) memcpy(occluded, d_occ, n);
+    }
     if (rc != YAR_OK) return rc;
     if (kernel_ms) {
         e = cudaEventElapsedTime(kernel_ms, ctx->ev_start, ctx->ev_stop);

@@ -90,6 +90,8 @@ struct yar_gpu_ctx {
     uint32_t staging_capacity = 0;
     yar::Device_Buffer d_rays, d_t, d_prim, d_obj, d_bary, d_occ;
     yar::Device_Buffer d_answers;  // the wide tree's answers of a cast
+    // page-locked host block for what small synchronous calls move (pinned_block)
+    char* pinned = nullptr;
     int* d_error = nullptr;  // device error word (stack overflow, bounded-wait expiry)
     uint32_t* d_counter = nullptr;  // ray hand-out counters of the persistent cast kernels, one per pipeline chunk
     // host-buffer casts in chunks: copies in, the traversal on two compute
@@ -137,6 +139,16 @@ namespace yar {
 
 int fail(yar_gpu_ctx* ctx, int code, const std::string& message);
 int cuda_fail(yar_gpu_ctx* ctx, cudaError_t e, const char* what);
+// The context's page-locked block (null without memory for it): two result
+// words, then the rays and results of a small host-buffer cast, which the
+// kernels write there themselves.  A copy from or to pageable memory holds the
+// host up until it is through, 8 us each.  Closest-hit casts from host arrays
+// with one such copy per array and with none: 64 rays 84 and 49 us, 1,021 99
+// and 64, 8,192 122 and 96, 16,384 135 and 128, 65,536 160 and 315 (the kernels'
+// 4-byte stores across the link).
+constexpr uint32_t kSmallCastRays = 8192;
+constexpr size_t kPinnedHead = 64;
+char* pinned_block(yar_gpu_ctx* ctx);
 int device_alloc(yar_gpu_ctx* ctx, Device_Buffer& b, size_t bytes);
 void device_free(Device_Buffer& b);
 

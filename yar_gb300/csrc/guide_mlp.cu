@@ -809,16 +809,19 @@ int guide_call_prologue(yar_gpu_ctx* ctx) {
 }
 
 int guide_finish(yar_gpu_ctx* ctx, cudaError_t e, const char* what, float* loss) {
+    struct {
+        int err;
+        float loss;
+    } h = {0, 0.f}, *words = &h;  // (pageable without the context's page-locked block)
+    if (char* p = pinned_block(ctx)) words = reinterpret_cast<decltype(words)>(p);
+    if (e == cudaSuccess && loss)
+        e = cudaMemcpyAsync(&words->loss, ctx->guide.scalars.ptr, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(&words->err, ctx->d_error, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, what);
-    if (loss) {
-        e = cudaMemcpy(loss, ctx->guide.scalars.ptr, sizeof(float), cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, what);
-    }
-    int h = 0;
-    e = cudaMemcpy(&h, ctx->d_error, sizeof(int), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, what);
-    if (h) {
+    if (loss) *loss = words->loss;
+    if (words->err) {
         cudaMemset(ctx->d_error, 0, sizeof(int));
         return fail(ctx, YAR_ERR_TIMEOUT, "tensor-core wait gave up");
     }
