@@ -373,7 +373,7 @@ typedef struct yar_hit_soa {
 typedef struct yar_gpu_options {
     int32_t device;                 /* CUDA device ordinal */
     uint32_t max_batch_rays;        /* capacity of the host-buffer staging area (0 = 16M) */
-    int32_t traversal_kernel;       /* YAR_TRAVERSAL_*: 0 = chosen per scene by timing */
+    int32_t traversal_kernel;       /* YAR_TRAVERSAL_*: 0 = chosen per scene */
     uint32_t pipeline_chunk_rays;   /* host-buffer casts of two or more chunks of this many rays (0 = 4M,
                                        at most 32 chunks) overlap their copies with the traversal once
                                        the traversal kernel is chosen; UINT32_MAX: never */
@@ -383,9 +383,9 @@ typedef struct yar_gpu_options {
  * whose objects are at most translated is cast through an 8-wide tree that the
  * upload builds; every hit is settled against the kd-tree, and rays it does not
  * settle walk the kd-tree one per thread (renders of scenes of tessellated
- * axis-parallel planes walk it for every ray): both are reported as PER_RAY.
- * The others, fixed by the options or chosen for scenes with rotated or scaled
- * objects, walk the kd-tree: persistent warps
+ * axis-parallel planes walk it for every ray, as PER_RAY).
+ * The others, fixed by the options or chosen for scenes without such a tree
+ * (a rotated or scaled object leaves it out), walk the kd-tree: persistent warps
  * at high occupancy (PERSISTENT_64: a register cap for 8 blocks of 128
  * threads per SM, 64 registers, for closest-hit rays and for 12 blocks, 40
  * registers, for any-hit rays), persistent warps with up to 128 registers
@@ -398,8 +398,10 @@ typedef struct yar_gpu_options {
 #define YAR_TRAVERSAL_PER_RAY 3
 #define YAR_TRAVERSAL_PER_RAY_VOTE 4  /* one ray per thread, the warp runs one traversal mode per iteration */
 
-/* The traversal kernels chosen so far on the uploaded scene (YAR_TRAVERSAL_*,
- * 0 = not chosen yet): cast[0] closest-hit and cast[1] any-hit C-ABI casts;
+/* The traversal kernels chosen so far on the uploaded scene (YAR_TRAVERSAL_*;
+ * AUTO, 0, where nothing has been timed and where AUTO's wide tree casts, which
+ * no other value of the option selects): cast[0] closest-hit and cast[1] any-hit
+ * C-ABI casts;
  * render_closest[b] / render_any[b] the render's extend and shadow queues of
  * bounce b (the last entry covers deeper bounces). */
 #define YAR_TRAVERSAL_BOUNCE_BUCKETS 5
@@ -495,7 +497,8 @@ typedef struct yar_batch_scene_stats {
     double variance;              /* render_scene's variance_estimate */
     float completion_seconds;     /* batch start to this scene's resolved film, GPU clock */
     uint64_t paths;               /* camera paths */
-    uint32_t traversal_kernel[2]; /* YAR_TRAVERSAL_* used for closest-hit and any-hit rays (as yar_gpu_traversal_kernels) */
+    uint32_t traversal_kernel[2]; /* YAR_TRAVERSAL_* used for closest-hit and any-hit rays (PER_RAY also
+                                     where the wide tree casts: AUTO selects that one) */
 } yar_batch_scene_stats;
 
 typedef struct yar_batch_stats {

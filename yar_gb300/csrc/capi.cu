@@ -116,9 +116,10 @@ extern "C" int yar_gpu_traversal_kernels(yar_gpu_ctx* ctx, int32_t cast[2], int3
                                          int32_t render_any[5]) {
     if (!ctx || !cast || !render_closest || !render_any) return YAR_ERR_INVALID;
     static_assert(yar_gpu_ctx::kBounceBuckets == YAR_TRAVERSAL_BOUNCE_BUCKETS, "bucket count");
-    // the wide tree's rays that it does not settle walk the kd-tree one per thread
+    // The wide tree has no value of its own: AUTO is the option that selects it
+    // (a context fixed to PER_RAY would walk the kd-tree, four times slower).
     auto code = [](int k) {
-        return k < 0 ? 0 : k == kCastWide ? YAR_TRAVERSAL_PER_RAY : k + YAR_TRAVERSAL_PERSISTENT_64;
+        return k < 0 || k == kCastWide ? YAR_TRAVERSAL_AUTO : k + YAR_TRAVERSAL_PERSISTENT_64;
     };
     for (int i = 0; i < 2; i++) cast[i] = code(ctx->cast_kernel[i]);
     for (int b = 0; b < yar_gpu_ctx::kBounceBuckets; b++) {

@@ -428,7 +428,8 @@ class Context:
 
     def traversal_kernels(self):
         """The traversal kernels chosen so far: {"cast": [closest, any], "render_closest": [per bounce],
-        "render_any": [per bounce]} as TRAVERSAL_* codes (0 = not chosen yet)."""
+        "render_any": [per bounce]} as TRAVERSAL_* codes (0, TRAVERSAL_AUTO: nothing timed, or the wide
+        tree casts)."""
         c, rc, ra = (C.c_int32 * 2)(), (C.c_int32 * 5)(), (C.c_int32 * 5)()
         self._check(lib().yar_gpu_traversal_kernels(self._h, c, rc, ra), "traversal_kernels")
         return {"cast": list(c), "render_closest": list(rc), "render_any": list(ra)}
