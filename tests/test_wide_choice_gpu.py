@@ -8,7 +8,7 @@ import pytest
 from conftest import cuda_available, golden
 from test_wide_gpu import assert_settled, probing_rays, soup
 from yar_gb300 import native, scenes
-from yar_gb300.scene import FlatScene
+from yar_gb300.scene import FlatScene, Mesh, make_object
 
 pytestmark = pytest.mark.gpu
 
@@ -40,3 +40,56 @@ def test_reported_kernels_select_what_ran():
     """The wide tree is reported as AUTO, a timed kd-tree kernel as itself."""
     assert casts_through_wide_tree(soup(5000, 21))
     assert not casts_through_wide_tree(FlatScene.read(golden("transform_small.yfs")))
+
+
+def flat_scene(triangles):
+    """One untransformed mesh of the triangles [n, 3, 3]."""
+    s = FlatScene()
+    p = np.asarray(triangles, np.float32)
+    s.meshes.append(Mesh(p.reshape(-1, 3), np.arange(3 * len(p)).reshape(-1, 3)))
+    m = np.eye(3, 4, dtype=np.float32).ravel()
+    s.objects = np.array([make_object(0, m, m)])
+    s.build_kdtrees(1)
+    return s
+
+
+def unit_cube():
+    c = np.array([[x, y, z] for x in (0, 1) for y in (0, 1) for z in (0, 1)], np.float64)
+    quads = [(0, 1, 3, 2), (4, 5, 7, 6), (0, 1, 5, 4), (2, 3, 7, 6), (0, 2, 6, 4), (1, 3, 7, 5)]
+    return np.array([[c[q[0]], c[q[k]], c[q[k + 1]]] for q in quads for k in (1, 2)])
+
+
+def fence():  # 2,000 equal cubes in a row
+    return unit_cube()[None] + 2.0 * np.arange(2000)[:, None, None, None] * np.array([1.0, 0, 0])
+
+
+def strip():  # 10,000 equal cells of a plane in a row
+    cell = np.array([[[0, 0, 0], [1, 0, 0], [1, 1, 0]], [[0, 0, 0], [1, 1, 0], [0, 1, 0]]], np.float64)
+    return cell[None] + np.arange(10000)[:, None, None, None] * np.array([1.0, 0, 0])
+
+
+def copies():  # 1,500 triangles of one box among random ones
+    rng = np.random.default_rng(31)
+    p = rng.random((20000, 1, 3)) + 0.02 * (rng.random((20000, 3, 3)) - 0.5)
+    p[7000:8500] = p[7000]
+    p[7000:8500, 1, 2] += np.linspace(0, 1, 1500) * (p[7000, 2, 2] - p[7000, 1, 2])
+    return p
+
+
+def growing():  # each half a percent larger than the one before it and past its end
+    k = 1.005 ** np.arange(3000)
+    base = np.array([[0, 0, 0], [1, 0, 0.2], [0.3, 1, 0.4]])
+    return k[:, None, None] * base + 210.0 * k[:, None, None] * np.array([1.0, 0, 0])
+
+
+@pytest.mark.parametrize("make", [fence, strip, copies, growing])
+def test_equal_and_growing_boxes(make):
+    """Neighbours of equal area, and boxes that grow along the builder's order,
+    above and below the cluster count that one block finishes: the tree is
+    built, and its casts are the kd-tree's."""
+    s = flat_scene(make().reshape(-1, 3, 3))
+    assert casts_through_wide_tree(s)
+    assert_settled(s, probing_rays(s, 32768, 32))
+    small = flat_scene(make().reshape(-1, 3, 3)[:1000])
+    assert casts_through_wide_tree(small)
+    assert_settled(small, probing_rays(small, 16384, 33))

@@ -8,7 +8,8 @@
 //   pairs    bottom-up clustering over the sorted order: every cluster finds
 //            the neighbour within kReach places whose union box has the least
 //            area, mutual choices merge, the survivors are compacted (parallel
-//            locally-ordered clustering, Meister and Bittner, TVCG 2018); from
+//            locally-ordered clustering, Meister and Bittner, TVCG 2018); after
+//            a round that merged few, neighbours in the order are paired; from
 //            kSmall clusters on, one block finishes
 //   costs    bottom up, which nodes of the pair tree become wide nodes, which
 //            joins of two triangles leaf children, by least expected cost
@@ -33,9 +34,15 @@ namespace {
 constexpr int kBuildBlock = 256;
 constexpr int kReach = 16;    // neighbours searched on either side (8, 32 and 64: the same casts within 2%)
 constexpr int kSmall = 1024;  // clusters one block finishes
-// Rounds of merging before a scene is left to the kd-tree (2.4M triangles take
-// about 40; boxes that grow steadily along the order could merge one pair a round).
-constexpr int kMaxRounds = 256;
+// A round of merging that takes in fewer than 1/16 of the clusters (2.4M
+// triangles merge about 1/6 a round) is followed by one that pairs every two
+// neighbours in the order.  Copies of one box, rows of equal cells and boxes
+// that grow steadily along the order choose each other one pair a round: 24,000
+// triangles of equal cubes in a row were not through after 256 rounds, 11.0 ms;
+// their upload now takes 1.9 ms.  (Breaking ties by the lesser XOR of the two
+// places, so that equal neighbours pair up by themselves: 1.6 ms, but the
+// 4.1M-triangle render takes 74.5 ms on that tree, 73.9 ms on this one.)
+constexpr uint32_t kFewMerges = 16;
 constexpr uint32_t kInnerBit = 0x80000000u;
 
 constexpr uint32_t kPlanarTriangles = 16384;  // of a scene of tessellated planes (yar_gpu_ctx::wide_planar)
@@ -322,9 +329,16 @@ wide_leaves_kernel(const float4* __restrict__ lo_in, const float4* __restrict__ 
 }
 
 // The nearest neighbour of each cluster within kReach places: least area of the
-// union, the lower place on equal areas (so a least pair is always mutual).
+// union, the lower place on equal areas (so a least pair is always mutual);
+// `pair` pairs neighbours in the order instead.
 __global__ void __launch_bounds__(kBuildBlock)
-wide_nearest_kernel(const float4* __restrict__ lo, const float4* __restrict__ hi, uint32_t n, uint32_t* __restrict__ nearest) {
+wide_nearest_kernel(const float4* __restrict__ lo, const float4* __restrict__ hi, uint32_t n, bool pair,
+                    uint32_t* __restrict__ nearest) {
+    if (pair) {
+        const uint32_t i = blockIdx.x * kBuildBlock + threadIdx.x;
+        if (i < n) nearest[i] = min(i ^ 1u, n - 1u);
+        return;
+    }
     __shared__ float box[6][kBuildBlock + 2 * kReach];
     const int first = (int)(blockIdx.x * kBuildBlock) - kReach;
     for (int k = threadIdx.x; k < kBuildBlock + 2 * kReach; k += kBuildBlock) {
@@ -432,8 +446,11 @@ wide_finish_kernel(const float4* __restrict__ lo, const float4* __restrict__ hi,
     if (i < n) box[i] = load_cluster(lo, hi, i);
     __syncthreads();
     uint32_t inner = inner_base;
+    bool pair = false;
     while (n > 1u) {  // each round merges at least the least pair
-        if (i < n) {
+        if (pair) {
+            if (i < n) nearest[i] = min(i ^ 1u, n - 1u);
+        } else if (i < n) {
             const Cluster c = box[i];
             float best = __int_as_float(0x7f800000);
             uint32_t at = i;
@@ -473,6 +490,7 @@ wide_finish_kernel(const float4* __restrict__ lo, const float4* __restrict__ hi,
         if (f == 2) c = merge_clusters(c, other, id, tree);
         if (f != 0) box[to] = c;
         if (total_m == 0u) break;  // (cannot happen with finite boxes)
+        pair = total_m * kFewMerges < n;
         n = total_s;
         inner += total_m;
         __syncthreads();
@@ -992,10 +1010,10 @@ cudaError_t wide_build(yar_gpu_ctx* ctx, const yar_flat_scene* scene, const uint
     uint32_t inner = 0;
     int side = 0;
     uint32_t* nearest = index[cur ^ 1];
-    for (int round = 0; n > (uint32_t)kSmall; round++) {
-        if (round == kMaxRounds) return cudaSuccess;
+    bool pair = false;
+    while (n > (uint32_t)kSmall) {
         const uint32_t b = (n + kBuildBlock - 1) / kBuildBlock;
-        wide_nearest_kernel<<<b, kBuildBlock, 0, st>>>(c_lo[side], c_hi[side], n, nearest);
+        wide_nearest_kernel<<<b, kBuildBlock, 0, st>>>(c_lo[side], c_hi[side], n, pair, nearest);
         wide_count_kernel<<<b, kBuildBlock, 0, st>>>(nearest, n, counts, counts + blocks);
         wide_scan_kernel<<<1, 1024, 0, st>>>(counts, b, words);
         wide_scan_kernel<<<1, 1024, 0, st>>>(counts + blocks, b, words + 1);
@@ -1007,6 +1025,7 @@ cudaError_t wide_build(yar_gpu_ctx* ctx, const yar_flat_scene* scene, const uint
         if (e != cudaSuccess) return e;
         const uint32_t stays = sums[0], merged = sums[1];
         if (merged == 0u) return cudaSuccess;  // (cannot happen with finite boxes)
+        pair = (uint64_t)merged * kFewMerges < n;
         n = stays;
         inner += merged;
         side ^= 1;
