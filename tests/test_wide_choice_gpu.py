@@ -93,3 +93,26 @@ def test_equal_and_growing_boxes(make):
     small = flat_scene(make().reshape(-1, 3, 3)[:1000])
     assert casts_through_wide_tree(small)
     assert_settled(small, probing_rays(small, 16384, 33))
+
+
+def test_launches_of_a_planar_scene():
+    """Renders of a scene of tessellated planes walk the kd-tree, one kernel a
+    cast: as many launches as with that kernel fixed, the same image."""
+    torch = pytest.importorskip("torch")
+    s = scenes.hard_lighting_room(cells=64)  # 49,000 triangles of axis-parallel planes
+    s.config["render_region"] = (0, 0, 64, 64)
+    got = []
+    for kernel in (native.TRAVERSAL_AUTO, native.TRAVERSAL_PER_RAY):
+        ctx = native.Context(0, traversal_kernel=kernel)
+        try:
+            ctx.upload_scene(s)
+            assert ctx.traversal_kernels()["render_closest"] == [native.TRAVERSAL_PER_RAY] * 5
+            ctx.render(64, 64)
+            img, stats = ctx.render(64, 64)  # the second one: bounces driven from the device
+            out = torch.zeros((64, 64, 3), dtype=torch.float32, device="cuda")
+            torch.cuda.synchronize()
+            static = ctx.render_static(out.data_ptr())
+            got.append((img.tobytes(), stats.kernel_launches, static.kernel_launches))
+        finally:
+            ctx.close()
+    assert got[0] == got[1]

@@ -654,7 +654,6 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
                                                                     q.ext_rays[from ^ 1], q.ext_slot[from ^ 1],
                                                                     ray_keys, ray_hist, count_dev, count);
     };
-    const uint32_t settles = ctx->ds.wide_nodes ? 3u : 0u;  // the wide tree's casts are two kernels each
     // The bounce loop over extend queue 0 of `count` paths; bounce0 picks the
     // traversal kernels.  Sets e; returns a YAR_ERR_* for a traversal overflow.
     auto run_bounces = [&](const Render_Params& pp, uint32_t count, int bounce0) -> int {
@@ -687,7 +686,7 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
             e = trace_light_queues(ctx, q, ps, count, bounce, st);
             if (e != cudaSuccess) break;
             connect_kernel<<<grid_for(count), kBlock, 0, st>>>(pp, S, q.ext_slot[cur], count, ps, nullptr);
-            launches += (mixed ? 7 : 5) + settles;
+            launches += (mixed ? 4 : 2) + cast_launches(ctx, bounce);
             uint32_t h[4];
             e = cudaMemcpyAsync(h, q.counters, sizeof(h), cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -758,7 +757,7 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
             e = launch_extend(ctx->ds, pr, render_choice(ctx, 0, bounce), st);
             if (e != cudaSuccess) break;
             connect_kernel<<<grid, kBlock, 0, st>>>(pp, S, q.ext_slot[cur], max_paths, ps, nullptr, q.counters + 7);
-            launches += (mixed ? 8 : 6) + settles;
+            launches += (mixed ? 5 : 3) + cast_launches(ctx, bounce);
             cur ^= 1;
         }
         bounce_begin_kernel<<<1, 1, 0, st>>>(q.counters, 0u, rays_dev);  // adds the last bounce's rays
@@ -1055,7 +1054,7 @@ int render_run_static(yar_gpu_ctx* ctx, float* rgb_out_device, yar_render_stats*
             e = trace_light_queues(ctx, q, ps, count, bounce, st);
             if (e != cudaSuccess) break;
             connect_kernel<<<grid_for(count), kBlock, 0, st>>>(pp, S, q.ext_slot[cur], count, ps, nullptr);
-            launches += 5 + (ctx->ds.wide_nodes ? 3 : 0);
+            launches += 2 + cast_launches(ctx, bounce);
             uint32_t h[4];
             e = cudaMemcpyAsync(h, q.counters, sizeof(h), cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);

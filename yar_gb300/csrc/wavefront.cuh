@@ -548,7 +548,12 @@ inline int bounce_bucket(int bounce) { return bounce < yar_gpu_ctx::kBounceBucke
 inline int render_choice(const yar_gpu_ctx* ctx, int kind, int bounce) {
     for (int b = bounce_bucket(bounce); b >= 0; b--)
         if (ctx->render_kernel[kind][b] >= 0) return ctx->render_kernel[kind][b];
-    return ctx->ds.wide_nodes ? kCastWide : kCastPersistent64;
+    return kCastPersistent64;
+}
+// Launches of a bounce's three casts (extend, shadow, probe): one each, two
+// through the wide tree.
+inline uint32_t cast_launches(const yar_gpu_ctx* ctx, int bounce) {
+    return 3u + (render_choice(ctx, 0, bounce) == kCastWide ? 2u : 0u) + (render_choice(ctx, 1, bounce) == kCastWide ? 1u : 0u);
 }
 
 cudaError_t trace_extend(yar_gpu_ctx* ctx, const Queues& q, int cur, uint32_t count, int bounce, cudaStream_t st) {
