@@ -426,9 +426,15 @@ void* yar_gpu_stream(yar_gpu_ctx* ctx);
 int yar_gpu_synchronize(yar_gpu_ctx* ctx);
 
 /* ---- scene ---- */
+/* Besides the kd-trees, an upload with traversal_kernel AUTO keeps the wide tree
+ * on the device, where the scene allows one.  A call that finds no memory for
+ * its buffers frees it (and a cast without memory for its answers leaves it
+ * aside); results are the same. */
 int yar_gpu_upload_scene(yar_gpu_ctx* ctx, const yar_flat_scene* scene);
 
-/* ---- ray casts (KdTree::intersect / intersect_any over the scene tree) ---- */
+/* ---- ray casts (KdTree::intersect / intersect_any over the scene tree) ----
+ * Casts through the wide tree, from device buffers too, keep 4 bytes per ray of
+ * the largest batch in the context. */
 int yar_gpu_cast_closest(yar_gpu_ctx* ctx, const yar_ray* rays, uint32_t ray_count,
                          const yar_hit_soa* hits, int32_t buffers);
 int yar_gpu_cast_any(yar_gpu_ctx* ctx, const yar_ray* rays, uint32_t ray_count,

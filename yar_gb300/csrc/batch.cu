@@ -92,10 +92,28 @@ struct Batch {
     }
 };
 
+// As work_alloc, with the trees of every scene of the batch (no graph of it is
+// running); `call` is repeated if they made room.
+template <class CALL>
+int with_room(Batch& bt, CALL call) {
+    int rc = call();
+    if (rc != YAR_ERR_NOMEM) return rc;
+    bool left = wide_leave(bt.ctx);
+    for (Batch_Scene& s : bt.scenes)
+        if (s.sub && wide_leave(s.sub)) {
+            left = true;
+            for (int& k : s.kernel)
+                if (k == kCastWide) k = kCastPersistent64;
+        }
+    return left ? call() : rc;
+}
+int batch_alloc(Batch& bt, Device_Buffer& b, size_t bytes) {
+    return with_room(bt, [&] { return device_alloc(bt.ctx, b, bytes); });
+}
+
 constexpr uint32_t kFixedGrid = 152 * 16;  // shade/connect grid when queue lengths live on the device
 
 int alloc_branches(Batch& bt, int nb, uint64_t chunk_cap, bool one_spp) {
-    yar_gpu_ctx* ctx = bt.ctx;
     for (Branch& b : bt.branches) {
         for (Device_Buffer& x : b.B) device_free(x);
         if (b.stream) cudaStreamDestroy(b.stream);
@@ -124,7 +142,7 @@ int alloc_branches(Batch& bt, int nb, uint64_t chunk_cap, bool one_spp) {
     int rc = YAR_OK;
     for (Branch& br : bt.branches) {
         cudaError_t e = cudaStreamCreateWithFlags(&br.stream, cudaStreamNonBlocking);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "batch streams");
+        if (e != cudaSuccess) return cuda_fail(bt.ctx, e, "batch streams");
         if (br.cap == 0) continue;
         br.B.assign(33, Device_Buffer{});
         const size_t cap = br.cap;
@@ -134,8 +152,8 @@ int alloc_branches(Batch& bt, int nb, uint64_t chunk_cap, bool one_spp) {
                                   cap * 8, cap * 32, cap * 4, cap * 32, cap * 4, 16 * sizeof(uint32_t),
                                   cap, cap * 4, 2 * kShadeClasses * sizeof(uint32_t),  // shading order
                                   cap * 2, kRayBins * sizeof(uint32_t)};              // extend-queue sort
-        for (int i = 2; i < 32 && rc == YAR_OK; i++) rc = device_alloc(ctx, br.B[i], sizes[i]);
-        if (br.diffs && rc == YAR_OK) rc = device_alloc(ctx, br.B[32], cap * 3 * sizeof(float4));
+        for (int i = 2; i < 32 && rc == YAR_OK; i++) rc = batch_alloc(bt, br.B[i], sizes[i]);
+        if (br.diffs && rc == YAR_OK) rc = batch_alloc(bt, br.B[32], cap * 3 * sizeof(float4));
         if (rc != YAR_OK) return rc;
         std::vector<Device_Buffer>& B = br.B;
         br.ps = Path_State{dp<float4>(B[4]), dp<float4>(B[5]), dp<uint32_t>(B[6]), dp<uint4>(B[7]),
@@ -359,7 +377,7 @@ int render_batch(yar_gpu_ctx* ctx, const yar_flat_scene* const* scenes, uint32_t
         Batch_Scene& s = bt.scenes[i];
         if (!scenes[i] || !rgb_out[i]) return fail(ctx, YAR_ERR_INVALID, "render batch: null scene or image");
         if ((rc = yar_gpu_create(&s.sub, &opt)) != YAR_OK) return fail(ctx, rc, "render batch: context");
-        if ((rc = yar_gpu_upload_scene(s.sub, scenes[i])) != YAR_OK)
+        if ((rc = with_room(bt, [&] { return yar_gpu_upload_scene(s.sub, scenes[i]); })) != YAR_OK)
             return fail(ctx, rc, "scene " + std::to_string(i) + ": " + yar_gpu_last_error(s.sub));
         if ((rc = prepare_render_params(s.sub, s.p)) != YAR_OK)
             return fail(ctx, rc, "scene " + std::to_string(i) + ": " + yar_gpu_last_error(s.sub));
@@ -369,16 +387,16 @@ int render_batch(yar_gpu_ctx* ctx, const yar_flat_scene* const* scenes, uint32_t
         s.pixels = (uint64_t)s.p.sw * s.p.sh;
         s.samples = s.pixels * s.p.spp;
         if (s.samples > 0xffffffffull) return fail(ctx, YAR_ERR_CAPACITY, "render batch: too many samples in a scene");
-        if ((rc = device_alloc(ctx, s.radiance, s.samples * sizeof(float4))) != YAR_OK) return rc;
-        if ((rc = device_alloc(ctx, s.image_samples, s.samples * sizeof(float2))) != YAR_OK) return rc;
-        if ((rc = device_alloc(ctx, s.pixel_var, pixel_film_bytes(s.pixels))) != YAR_OK) return rc;
-        if ((rc = device_alloc(ctx, s.tile_var, (size_t)s.p.tiles_x * s.p.tiles_y * sizeof(double))) != YAR_OK)
+        if ((rc = batch_alloc(bt, s.radiance, s.samples * sizeof(float4))) != YAR_OK) return rc;
+        if ((rc = batch_alloc(bt, s.image_samples, s.samples * sizeof(float2))) != YAR_OK) return rc;
+        if ((rc = batch_alloc(bt, s.pixel_var, pixel_film_bytes(s.pixels))) != YAR_OK) return rc;
+        if ((rc = batch_alloc(bt, s.tile_var, (size_t)s.p.tiles_x * s.p.tiles_y * sizeof(double))) != YAR_OK)
             return rc;
-        if ((rc = device_alloc(ctx, s.variance, sizeof(double))) != YAR_OK) return rc;
-        if ((rc = device_alloc(ctx, s.rgb, (size_t)s.p.rw * s.p.rh * 3 * sizeof(float))) != YAR_OK) return rc;
+        if ((rc = batch_alloc(bt, s.variance, sizeof(double))) != YAR_OK) return rc;
+        if ((rc = batch_alloc(bt, s.rgb, (size_t)s.p.rw * s.p.rh * 3 * sizeof(float))) != YAR_OK) return rc;
     }
-    if ((rc = device_alloc(ctx, bt.stamps, (1 + count) * sizeof(unsigned long long))) != YAR_OK) return rc;
-    if ((rc = device_alloc(ctx, bt.rays, 2 * 16 * sizeof(unsigned long long))) != YAR_OK) return rc;
+    if ((rc = batch_alloc(bt, bt.stamps, (1 + count) * sizeof(unsigned long long))) != YAR_OK) return rc;
+    if ((rc = batch_alloc(bt, bt.rays, 2 * 16 * sizeof(unsigned long long))) != YAR_OK) return rc;
     const double upload_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
 
     // autotuner, step 1: traversal kernel per scene on random rays in its box
@@ -386,8 +404,8 @@ int render_batch(yar_gpu_ctx* ctx, const yar_flat_scene* const* scenes, uint32_t
     {
         Device_Buffer rays_buf, hits;
         const uint32_t n = 1u << 16;
-        if ((rc = device_alloc(ctx, rays_buf, (size_t)n * 32)) != YAR_OK) return rc;
-        if ((rc = device_alloc(ctx, hits, (size_t)n * 24)) != YAR_OK) return rc;
+        if ((rc = batch_alloc(bt, rays_buf, (size_t)n * 32)) != YAR_OK) return rc;
+        if ((rc = batch_alloc(bt, hits, (size_t)n * 24)) != YAR_OK) return rc;
         cudaError_t e = cudaSuccess;
         for (uint32_t i = 0; i < count && e == cudaSuccess; i++) {
             Batch_Scene& s = bt.scenes[i];

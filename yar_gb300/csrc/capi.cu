@@ -42,6 +42,24 @@ int device_alloc(yar_gpu_ctx* ctx, Device_Buffer& b, size_t bytes) {
     return YAR_OK;
 }
 
+bool wide_leave(yar_gpu_ctx* ctx) {
+    if (!ctx->ds.wide_nodes) return false;
+    cudaStreamSynchronize(ctx->stream);
+    wide_release(ctx);
+    device_free(ctx->d_answers);
+    for (int k = 0; k < 2; k++) {
+        ctx->cast_kernel[k] = -1;  // (a scene with a wide tree has no fixed kernel)
+        for (int& b : ctx->render_kernel[k]) b = -1;
+    }
+    ctx->render_tuned = false;
+    return true;
+}
+
+int work_alloc(yar_gpu_ctx* ctx, Device_Buffer& b, size_t bytes) {
+    const int rc = device_alloc(ctx, b, bytes);
+    return rc == YAR_ERR_NOMEM && wide_leave(ctx) ? device_alloc(ctx, b, bytes) : rc;
+}
+
 char* pinned_block(yar_gpu_ctx* ctx) {
     if (!ctx->pinned) {
         void* p = nullptr;
@@ -337,6 +355,11 @@ extern "C" int yar_gpu_upload_scene(yar_gpu_ctx* ctx, const yar_flat_scene* scen
     int fixed = ctx->forced_kernel;
     if (fixed < 0) {
         e = wide_build(ctx, scene, tri_offset.data(), node_offset.data());
+        if (e == cudaErrorMemoryAllocation) {  // (a launch's local memory)
+            cudaGetLastError();
+            wide_release(ctx);
+            e = cudaSuccess;
+        }
         if (e != cudaSuccess) return cuda_fail(ctx, e, "wide tree build");
         if (ds.wide_nodes) fixed = kCastWide;
     }
@@ -357,14 +380,14 @@ int ensure_staging(yar_gpu_ctx* ctx, uint32_t n, bool closest) {
     if (n > ctx->staging_capacity)
         return fail(ctx, YAR_ERR_CAPACITY, "batch of " + std::to_string(n) + " rays exceeds max_batch_rays");
     int rc;
-    if (ctx->d_rays.bytes < (size_t)n * 32 && (rc = device_alloc(ctx, ctx->d_rays, (size_t)n * 32)) != YAR_OK) return rc;
+    if (ctx->d_rays.bytes < (size_t)n * 32 && (rc = work_alloc(ctx, ctx->d_rays, (size_t)n * 32)) != YAR_OK) return rc;
     if (closest) {
-        if (ctx->d_t.bytes < (size_t)n * 4 && (rc = device_alloc(ctx, ctx->d_t, (size_t)n * 4)) != YAR_OK) return rc;
-        if (ctx->d_prim.bytes < (size_t)n * 4 && (rc = device_alloc(ctx, ctx->d_prim, (size_t)n * 4)) != YAR_OK) return rc;
-        if (ctx->d_obj.bytes < (size_t)n * 4 && (rc = device_alloc(ctx, ctx->d_obj, (size_t)n * 4)) != YAR_OK) return rc;
-        if (ctx->d_bary.bytes < (size_t)n * 8 && (rc = device_alloc(ctx, ctx->d_bary, (size_t)n * 8)) != YAR_OK) return rc;
+        if (ctx->d_t.bytes < (size_t)n * 4 && (rc = work_alloc(ctx, ctx->d_t, (size_t)n * 4)) != YAR_OK) return rc;
+        if (ctx->d_prim.bytes < (size_t)n * 4 && (rc = work_alloc(ctx, ctx->d_prim, (size_t)n * 4)) != YAR_OK) return rc;
+        if (ctx->d_obj.bytes < (size_t)n * 4 && (rc = work_alloc(ctx, ctx->d_obj, (size_t)n * 4)) != YAR_OK) return rc;
+        if (ctx->d_bary.bytes < (size_t)n * 8 && (rc = work_alloc(ctx, ctx->d_bary, (size_t)n * 8)) != YAR_OK) return rc;
     } else {
-        if (ctx->d_occ.bytes < (size_t)n && (rc = device_alloc(ctx, ctx->d_occ, (size_t)n)) != YAR_OK) return rc;
+        if (ctx->d_occ.bytes < (size_t)n && (rc = work_alloc(ctx, ctx->d_occ, (size_t)n)) != YAR_OK) return rc;
     }
     return YAR_OK;
 }
@@ -497,6 +520,10 @@ int cast(yar_gpu_ctx* ctx, const yar_ray* rays, uint32_t n, const yar_hit_soa* h
     if (n == 0) return YAR_OK;
     cudaSetDevice(ctx->device);
     cudaError_t e;
+    if (buffers == YAR_BUFFERS_HOST) {
+        const int rc = ensure_staging(ctx, n, closest);
+        if (rc != YAR_OK) return rc;
+    }
     // The wide tree's answers, kept between calls.  Without memory for them a
     // cast uses the kd-tree kernel that untimed batches use.
     int wide_or_fixed = ctx->cast_kernel[closest ? 0 : 1];
@@ -510,8 +537,6 @@ int cast(yar_gpu_ctx* ctx, const yar_ray* rays, uint32_t n, const yar_hit_soa* h
     uint8_t* d_occ = nullptr;
     char* small = buffers == YAR_BUFFERS_HOST && n <= kSmallCastRays ? pinned_block(ctx) : nullptr;
     if (buffers == YAR_BUFFERS_HOST) {
-        int rc = ensure_staging(ctx, n, closest);
-        if (rc != YAR_OK) return rc;
         // a tuned (or fixed) traversal kernel and at least two chunks: overlap copies and traversal
         const int tuned = wide_or_fixed;
         if (!kernel_ms && pipeline_chunks(ctx, n) >= 2 && (tuned >= 0 || n < kTuneMinRays))

@@ -645,7 +645,8 @@ int render_direct(yar_gpu_ctx* ctx, float* rgb_out, yar_render_stats* stats) {
     for (int k = 0; k < env_samples; k++) units.push_back({kUnitEnvironment, 0, k, 1, 0, 0, env_samples, 0});
 
     // scratch: a buffer of the last call is kept when it is large enough;
-    // without the memory for a full chunk, smaller chunks
+    // without the memory for a full chunk, smaller chunks, and without the
+    // memory for the least one, the wide tree's
     std::vector<Device_Buffer>& B = ctx->render_scratch;
     if (B.size() != kDirectBuffers) {
         for (Device_Buffer& b : B) device_free(b);
@@ -657,7 +658,7 @@ int render_direct(yar_gpu_ctx* ctx, float* rgb_out, yar_render_stats* stats) {
     };
     uint64_t chunk_pixels = 0, cap = 0, slots = 0, per_launch = 0;
     const uint64_t most_units = std::max<uint64_t>(1, std::min<uint64_t>(units.size(), kMaxUnits));
-    for (uint64_t shrink = 1;; shrink *= 4) {
+    for (uint64_t shrink = 1;;) {
         rc = YAR_OK;
         chunk_pixels = std::max<uint64_t>(1, std::min<uint64_t>(pixels, kDirectPaths / shrink / p.spp));
         cap = chunk_pixels * p.spp;  // samples per chunk
@@ -696,8 +697,10 @@ int render_direct(yar_gpu_ctx* ctx, float* rgb_out, yar_render_stats* stats) {
         alloc(30, slots * sizeof(uint32_t));                  // probe and delta slots
         alloc(31, (env_samples ? 2 : 1) * slots * sizeof(uint32_t));    // the wide tree's answers
         alloc(32, 8 * sizeof(uint32_t));                      // queue counters, ray hand-out
-        if (rc != YAR_ERR_NOMEM || (chunk_pixels == 1 && per_launch == 1)) break;
+        const bool least = chunk_pixels == 1 && per_launch == 1;
+        if (rc != YAR_ERR_NOMEM || (least && !wide_leave(ctx))) break;
         for (Device_Buffer& b : B) device_free(b);
+        shrink = least ? 1 : 4 * shrink;
     }
     if (rc != YAR_OK) return rc;
     Path_State ps{};

@@ -677,12 +677,12 @@ int guide_ensure(yar_gpu_ctx* ctx) {
     const size_t pb = kGuideParams * sizeof(float);
     cudaSetDevice(ctx->device);
     if (sm_count() <= 0) return fail(ctx, YAR_ERR_INVALID, "guide: no SM count for the device");
-    if ((rc = device_alloc(ctx, g.params, pb)) != YAR_OK) return rc;
-    if ((rc = device_alloc(ctx, g.adam_m, pb)) != YAR_OK) return rc;
-    if ((rc = device_alloc(ctx, g.adam_v, pb)) != YAR_OK) return rc;
-    if ((rc = device_alloc(ctx, g.images, kImgBytes)) != YAR_OK) return rc;
-    if ((rc = device_alloc(ctx, g.partials, (size_t)sm_count() * pb)) != YAR_OK) return rc;
-    if ((rc = device_alloc(ctx, g.scalars, 64)) != YAR_OK) return rc;
+    if ((rc = work_alloc(ctx, g.params, pb)) != YAR_OK) return rc;
+    if ((rc = work_alloc(ctx, g.adam_m, pb)) != YAR_OK) return rc;
+    if ((rc = work_alloc(ctx, g.adam_v, pb)) != YAR_OK) return rc;
+    if ((rc = work_alloc(ctx, g.images, kImgBytes)) != YAR_OK) return rc;
+    if ((rc = work_alloc(ctx, g.partials, (size_t)sm_count() * pb)) != YAR_OK) return rc;
+    if ((rc = work_alloc(ctx, g.scalars, 64)) != YAR_OK) return rc;
     cudaError_t e = cudaMemsetAsync(g.images.ptr, 0, kImgBytes, ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "guide init");
     static bool attr[64] = {};  // per device

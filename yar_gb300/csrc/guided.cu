@@ -186,7 +186,7 @@ int guided_render(yar_gpu_ctx* ctx, const yar_guided_params* gp, double* sum_out
         B.assign(40, Device_Buffer{});
     }
     auto alloc = [&](int i, size_t bytes) {  // kept from an earlier call when large enough
-        if (rc == YAR_OK && bytes && !(B[i].ptr && B[i].bytes >= bytes)) rc = device_alloc(ctx, B[i], bytes);
+        if (rc == YAR_OK && bytes && !(B[i].ptr && B[i].bytes >= bytes)) rc = work_alloc(ctx, B[i], bytes);
     };
     const size_t cap = paths;
     alloc(1, cap * sizeof(float2));                        // image-plane samples
@@ -353,8 +353,8 @@ int guided_render(yar_gpu_ctx* ctx, const yar_guided_params* gp, double* sum_out
         if (guided) {
             const size_t qbytes = hook.chunk_paths * 3 * sizeof(float4);
             const size_t lbytes = hook.chunk_paths * kGuideLobeFloats * sizeof(float);
-            if (!(qbuf.ptr && qbuf.bytes >= qbytes)) rc = device_alloc(ctx, qbuf, qbytes);
-            if (rc == YAR_OK && !(lbuf.ptr && lbuf.bytes >= lbytes)) rc = device_alloc(ctx, lbuf, lbytes);
+            if (!(qbuf.ptr && qbuf.bytes >= qbytes)) rc = work_alloc(ctx, qbuf, qbytes);
+            if (rc == YAR_OK && !(lbuf.ptr && lbuf.bytes >= lbytes)) rc = work_alloc(ctx, lbuf, lbytes);
             if (rc != YAR_OK) return rc;
             hs.queries = dp<float4>(qbuf);
             hs.lobes = dp<float>(lbuf);

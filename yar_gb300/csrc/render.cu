@@ -516,7 +516,7 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
     }
     int rc = YAR_OK;
     auto alloc = [&](int i, size_t bytes) {
-        if (rc == YAR_OK && !(B[i].ptr && B[i].bytes >= bytes)) rc = device_alloc(ctx, B[i], bytes);
+        if (rc == YAR_OK && !(B[i].ptr && B[i].bytes >= bytes)) rc = work_alloc(ctx, B[i], bytes);
     };
     alloc(0, samples * sizeof(float4));                    // radiance
     alloc(1, samples * sizeof(float2));                    // image-plane samples
@@ -846,8 +846,8 @@ int render_run_params(yar_gpu_ctx* ctx, const Render_Params& p_in, float* rgb_ou
             max_area = std::max(max_area, area);
         }
         Device_Buffer offs, pix;
-        int rc2 = device_alloc(ctx, offs, tiles_out->offset.size() * sizeof(uint32_t));
-        if (rc2 == YAR_OK) rc2 = device_alloc(ctx, pix, std::max<size_t>(1, tiles_out->offset[n_tiles]) * sizeof(float4));
+        int rc2 = work_alloc(ctx, offs, tiles_out->offset.size() * sizeof(uint32_t));
+        if (rc2 == YAR_OK) rc2 = work_alloc(ctx, pix, std::max<size_t>(1, tiles_out->offset[n_tiles]) * sizeof(float4));
         if (rc2 != YAR_OK) {
             device_free(offs);
             device_free(pix);
