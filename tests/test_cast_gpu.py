@@ -344,3 +344,29 @@ def test_small_host_casts_match_device_casts(n):
         assert g.tobytes() == w.cpu().numpy().tobytes()
     assert np.array_equal(alone, got[2])
     ctx.close()
+
+
+def test_as_many_rays_as_the_interface_takes():
+    """2^32 - 1 any-hit rays on the device: the same 2^20 again and again."""
+    torch = pytest.importorskip("torch")
+    n, m = (1 << 32) - 1, 1 << 20
+    if torch.cuda.mem_get_info()[0] < 170 << 30:
+        pytest.skip("needs 170 GiB of free device memory")
+    s = scenes.raycast_scene(seed=2, grid=48, spheres=5, level=2)
+    lo, hi = scenes.scene_box(s)
+    few = scenes.random_shadow_rays(lo, hi, m, 45)
+    rays = torch.as_tensor(few).cuda().repeat(1 << 12, 1)
+    occ = torch.full((1 << 32,), 7, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    ctx = native.Context(0)
+    try:
+        ctx.upload_scene(s)
+        want = torch.as_tensor(ctx.cast_any(few)).cuda()
+        ctx.cast_any_device(rays.data_ptr(), n, occ.data_ptr())
+    finally:
+        ctx.close()
+    assert int(occ[-1]) == 7  # past the last ray
+    occ[-1] = want[-1]
+    assert bool((occ.view(-1, m) == want).all())
+    del rays, occ
+    torch.cuda.empty_cache()

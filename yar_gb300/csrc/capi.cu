@@ -17,6 +17,10 @@ namespace {
 // Casts of at least this many rays choose the traversal kernel by timing
 // (smaller batches use the persistent 64-register kernel until then).
 constexpr uint32_t kTuneMinRays = 1u << 20;
+// Rays per launch: the persistent kernels' hand-out word is 32 bits and passes
+// the last ray by a batch per warp (up to 1.3M rays); past 2^32 it would begin
+// again at the first ray, without end.
+constexpr uint32_t kMaxCastRays = 1u << 31;
 }  // namespace
 
 int fail(yar_gpu_ctx* ctx, int code, const std::string& message) {
@@ -377,8 +381,6 @@ extern "C" int yar_gpu_upload_scene(yar_gpu_ctx* ctx, const yar_flat_scene* scen
 namespace {
 
 int ensure_staging(yar_gpu_ctx* ctx, uint32_t n, bool closest) {
-    if (n > ctx->staging_capacity)
-        return fail(ctx, YAR_ERR_CAPACITY, "batch of " + std::to_string(n) + " rays exceeds max_batch_rays");
     int rc;
     if (ctx->d_rays.bytes < (size_t)n * 32 && (rc = work_alloc(ctx, ctx->d_rays, (size_t)n * 32)) != YAR_OK) return rc;
     if (closest) {
@@ -518,6 +520,22 @@ int cast(yar_gpu_ctx* ctx, const yar_ray* rays, uint32_t n, const yar_hit_soa* h
     if (!closest && n && !occluded) return fail(ctx, YAR_ERR_INVALID, "null output buffer");
     if (buffers != YAR_BUFFERS_HOST && buffers != YAR_BUFFERS_DEVICE) return fail(ctx, YAR_ERR_INVALID, "buffers flag");
     if (n == 0) return YAR_OK;
+    if (buffers == YAR_BUFFERS_HOST && n > ctx->staging_capacity)
+        return fail(ctx, YAR_ERR_CAPACITY, "batch of " + std::to_string(n) + " rays exceeds max_batch_rays");
+    if (n > kMaxCastRays) {
+        yar_hit_soa rest{};
+        if (closest)
+            rest = {hits->t ? hits->t + kMaxCastRays : nullptr, hits->prim ? hits->prim + kMaxCastRays : nullptr,
+                    hits->object ? hits->object + kMaxCastRays : nullptr,
+                    hits->bary ? hits->bary + 2 * (size_t)kMaxCastRays : nullptr};
+        float ms[2] = {0.f, 0.f};
+        int rc = cast(ctx, rays, kMaxCastRays, hits, occluded, buffers, kernel_ms ? &ms[0] : nullptr);
+        if (rc == YAR_OK)
+            rc = cast(ctx, rays + kMaxCastRays, n - kMaxCastRays, closest ? &rest : nullptr,
+                      closest ? nullptr : occluded + kMaxCastRays, buffers, kernel_ms ? &ms[1] : nullptr);
+        if (kernel_ms) *kernel_ms = ms[0] + ms[1];
+        return rc;
+    }
     cudaSetDevice(ctx->device);
     cudaError_t e;
     if (buffers == YAR_BUFFERS_HOST) {
