@@ -116,3 +116,34 @@ def test_launches_of_a_planar_scene():
         finally:
             ctx.close()
     assert got[0] == got[1]
+
+
+def moved(s, linear):
+    """The scene with its second object under one more linear part."""
+    o = s.objects[1]
+    m = np.asarray(o["object_to_world"], np.float64).reshape(3, 4)
+    m = np.concatenate([linear @ m[:, :3], m[:, 3:]], axis=1)
+    inv = np.linalg.inv(np.concatenate([m, [[0, 0, 0, 1]]]))[:3]
+    s.objects[1] = make_object(1, m.astype(np.float32).ravel(), inv.astype(np.float32).ravel())
+    s.build_kdtrees(1)
+    return s
+
+
+TURN = np.array([[0.8, -0.6, 0], [0.6, 0.8, 0], [0, 0, 1]])
+
+
+@pytest.mark.parametrize("make,wide", [
+    (lambda: soup(1, 1), True), (lambda: soup(1025, 2), True), (lambda: soup(3000, 5, 1e-6), True),
+    (lambda: soup(3000, 5, 1e6), True), (lambda: soup(3000, 5, 1.0, -30000.0), True),
+    (lambda: soup(2000, 7, copies=900), True), (lambda: scenes.hard_lighting_room(cells=24), True),
+    (lambda: FlatScene.read(golden("cornell_alpha_64.yfs")), True),
+    (lambda: soup(3000, 5, 1e-12), False), (lambda: soup(3000, 5, 1e12), False),
+    (lambda: moved(soup(3000, 5), TURN), False), (lambda: moved(soup(3000, 5), 1.5 * np.eye(3)), False)],
+    ids=["one", "1025", "small", "large", "far", "copies", "walls", "alpha", "too small", "too large",
+         "one of two rotated", "one of two scaled"])
+def test_which_scenes_have_a_wide_tree(make, wide):
+    """The scenes that the settling is tested on do cast through the tree, and
+    those that it does not take walk the kd-tree, with its results."""
+    s = make()
+    assert casts_through_wide_tree(s) == wide
+    assert_settled(s, probing_rays(s, 4096, 34))
