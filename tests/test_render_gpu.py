@@ -572,3 +572,20 @@ def test_render_c1_configuration_matches_the_reference(gpu_ctx):
     assert same >= BIT_EQUAL_MIN and rel < MEAN_REL_TOL, (same, rel)
     assert abs(stats.variance - float(g["variance"])) <= VARIANCE_REL_TOL * float(g["variance"])
     assert stats.paths == 256 * 256 * 16
+
+
+@pytest.mark.parametrize("maxb", [1, 2, 5, 9, 10, 11, 24])
+@pytest.mark.parametrize("name", ["cornell_delta_64", "cornell_mix_64", "cornell_c1_64"])
+def test_tail_waves_match_host_driven(gpu_ctx, name, maxb):
+    """The exact tail's waves leave out the bounces that a deferred path has
+    behind it; the host-driven loop stops at an empty queue instead.  Vertices
+    of three to five 1D dimensions, budgets of one vertex and of many."""
+    s = _past_budget_scene(name)
+    s.config["max_light_bounces"] = maxb
+    s.config["russian_roulette_bounce_count_threshold"] = 1
+    s.config["rng_seed_offset"] = maxb
+    gpu_ctx.upload_scene(s)
+    img1, st1 = gpu_ctx.render(64, 64)
+    img2, st2 = gpu_ctx.render(64, 64)
+    assert np.array_equal(img1.view(np.uint32), img2.view(np.uint32))
+    assert (st1.variance, st1.rays_closest, st1.rays_any) == (st2.variance, st2.rays_closest, st2.rays_any)
