@@ -7,8 +7,8 @@ the reference builder's algorithm; 16,777,216 closest-hit rays with origins
 uniform in the scene box and directions uniform on the sphere, and
 16,777,216 shadow rays with tmax = U[0,1] x |scene diagonal|.
 
-One step = one extend launch over the 16M rays + one shadow launch over the
-16M shadow rays.  metric = Mrays/s over both ray kinds.
+One step = one closest-hit call over the 16M rays + one any-hit call over the
+16M shadow rays, two kernels each.  metric = Mrays/s over both ray kinds.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl gb300|reference]
 
@@ -150,30 +150,34 @@ class ClockSampler:
                 "samples": len(sm)}
 
 
-# ------------------------------------------------------------------ algorithmic bytes
-def algorithmic_bytes(s, rays, shadow, sample=65536):
-    """Per-ray bytes of the traversal in the reference's visit order, counted by
-    the oracle on a sample of the same batches:
-      closest: 32 (ray) + 20 (hit) + 8*nodes + 4*leaf index words + 48*triangles + 96*object visits
-      any:     32 (ray) + 1 (bit)  + the same traversal terms
-    (48 B per triangle = 12 B indices + 36 B vertices; 96 B per object record)."""
-    import oracle
-    idx = np.linspace(0, rays.shape[0] - 1, sample).astype(np.int64)
-    _, _, _, _, st = oracle.cast_closest(s, rays[idx], with_stats=True)
-    _, st2 = oracle.cast_any(s, shadow[idx], with_stats=True)
-    w = np.array([8, 4, 48, 96], np.float64)
-    closest = 52.0 + (st.astype(np.float64) @ w).mean()
-    anyhit = 33.0 + (st2.astype(np.float64) @ w).mean()
-    return closest, anyhit, st.mean(0).tolist(), st2.mean(0).tolist()
+# ------------------------------------------------------------------ the casts' bytes
+def cast_bytes(triangles, rays):
+    """The bytes that a closest-hit and an any-hit batch cannot do without: each
+    ray (32 B) read and its result (20 B, 1 B) written once, and the scene's
+    triangles (36 B each) read once."""
+    return rays * (32 + 20) + 36 * triangles, rays * (32 + 1) + 36 * triangles
+
+
+def cast_roofline(triangles, rays, closest_ms, peak, peak_source):
+    """The closest-hit call against the copy bandwidth.  The casts are bound by
+    their issue slots, not by these bytes; the DRAM traffic is that of both
+    kernels of the call in the committed ncu summary, per ray."""
+    closest, anyhit = cast_bytes(triangles, rays)
+    achieved = closest / (closest_ms * 1e-3) / 1e9
+    per_ray = profile_traffic()
+    return {"bound": "issue", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
+            "frac": round(achieved / peak, 4), "peak_source": peak_source,
+            "traffic": None if per_ray is None else round(per_ray * rays), "kernel": "cast_wide + settle_wide",
+            "algorithmic_bytes_per_ray": round(closest / rays, 1), "any_hit_bytes_per_ray": round(anyhit / rays, 1)}
 
 
 def profile_traffic():
-    """DRAM bytes per extend launch from the committed ncu summary, if any."""
-    path = os.path.join(ROOT, "profiles", "extend_raycast_c2.md")
+    """DRAM bytes per closest-hit ray from the committed ncu summary, if any."""
+    path = os.path.join(ROOT, "profiles", "wide_cast_and_settle.md")
     if not os.path.exists(path):
         return None
     for ln in open(path):
-        if ln.startswith("traffic_bytes_per_launch:"):
+        if ln.startswith("traffic_bytes_per_ray:"):
             try:
                 return float(ln.split(":", 1)[1].strip())
             except ValueError:
@@ -446,7 +450,6 @@ def run_gb300(args, rank, world, local, pg):
         return
     ext_ms = statistics.median([a for a, b in kernel_times])
     shd_ms = statistics.median([b for a, b in kernel_times])
-    bpr_closest, bpr_any, st_c, st_a = algorithmic_bytes(s, rays, shadow)
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
@@ -454,8 +457,6 @@ def run_gb300(args, rank, world, local, pg):
         pass
     peak = peaks.get("hbm_gbs", 6800.0)
     peak_src = "measured" if "hbm_gbs" in peaks else "fallback"
-    achieved = bpr_closest * n / (ext_ms * 1e-3) / 1e9
-    traffic = profile_traffic()
     line = {
         "metric": METRIC, "value": round(value, 3), "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": round(ms_per_step, 3), "higher_is_better": True, "scaling": "weak",
@@ -464,18 +465,10 @@ def run_gb300(args, rank, world, local, pg):
         "config": raycast_config(s.triangle_count, n, world, args.grid),
         "e2e": {"value": round(e2e_value, 3), "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "pipeline_chunk_rays": 4 << 20, "host_copy_gbs": host_copy},
-        "gpu_launches": 2 * args.steps,
+        "gpu_launches": 4 * args.steps,  # cast_wide and settle_wide for each ray kind
         "kernels": {"extend_ms": round(ext_ms, 3), "shadow_ms": round(shd_ms, 3),
                     "extend_mrays_s": round(n / ext_ms / 1e3, 1), "shadow_mrays_s": round(n / shd_ms / 1e3, 1)},
-        "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                     "frac": round(achieved / peak, 4), "peak_source": peak_src,
-                     "traffic": traffic, "kernel": "extend",
-                     "algorithmic_bytes_per_ray": round(bpr_closest, 1),
-                     "any_hit_bytes_per_ray": round(bpr_any, 1),
-                     "mean_per_ray_closest": dict(zip(["nodes", "leaf_words", "triangles", "objects"],
-                                                      [round(x, 2) for x in st_c])),
-                     "mean_per_ray_any": dict(zip(["nodes", "leaf_words", "triangles", "objects"],
-                                                  [round(x, 2) for x in st_a]))},
+        "roofline": cast_roofline(s.triangle_count, n, ext_ms, peak, peak_src),
         "clocks": clocks.summary(),
         "setup": setup,
         "outputs_consistent": same,
@@ -559,7 +552,7 @@ def render_bench(kind, with_cpu=True, reps=3):
            "gpu_mrays_per_s": round((best.rays_closest + best.rays_any) / best.seconds / 1e6, 2),
            "rays_closest": int(best.rays_closest), "rays_any": int(best.rays_any),
            "kernel_launches": int(best.kernel_launches), "image_mean": float(img.mean()),
-           "traversal_kernels": {k: [["-", "p64", "p128", "per_ray", "per_ray_vote"][c] for c in v]
+           "traversal_kernels": {k: [["auto", "p64", "p128", "per_ray", "per_ray_vote"][c] for c in v]
                                  for k, v in kernels.items() if k != "cast"}}
     if not with_cpu:
         return out
