@@ -147,3 +147,80 @@ def test_which_scenes_have_a_wide_tree(make, wide):
     s = make()
     assert casts_through_wide_tree(s) == wide
     assert_settled(s, probing_rays(s, 4096, 34))
+
+
+def doubled(s, part):
+    """The scene with the first `part` of every mesh's triangles once more, their
+    vertices in another order."""
+    for m in s.meshes:
+        again = m.indices[:int(part * m.triangle_count)][:, [0, 2, 1]]
+        m.indices = np.concatenate([m.indices, again])
+    s.build_kdtrees(1)
+    return s
+
+
+@pytest.mark.parametrize("part,timed", [(0.0, False), (0.1, False), (0.3, True), (1.0, True)])
+def test_scenes_of_twins(part, timed):
+    """Where many triangles are there twice, closest hits (near ties) are timed
+    among the kd-tree kernels; shadow rays keep the wide tree."""
+    s = doubled(soup(3000, 41), part)
+    ctx = native.Context(0)
+    try:
+        ctx.upload_scene(s)
+        lo, hi = scenes.scene_box(s)
+        rays = scenes.random_rays(lo, hi, TIMED_RAYS, 62)
+        ctx.cast_closest(rays)
+        ctx.cast_any(rays)
+        kernels = ctx.traversal_kernels()["cast"]
+    finally:
+        ctx.close()
+    assert (kernels[0] != 0) == timed and kernels[1] == 0
+    assert_settled(s, probing_rays(s, 16384, 42))
+
+
+def test_twins_of_a_render():
+    s = FlatScene.read(golden("cornell_c1_64.yfs"))
+    s.config["render_region"] = (0, 0, 256, 256)
+    s.camera["image_extent"] = (256, 256)
+    s = doubled(s, 1.0)
+    got = []
+    for kernel in (native.TRAVERSAL_AUTO, native.TRAVERSAL_PER_RAY):
+        ctx = native.Context(0, traversal_kernel=kernel)
+        try:
+            ctx.upload_scene(s)
+            got += [ctx.render(256, 256) for _ in range(2)]
+            kernels = ctx.traversal_kernels()
+            if kernel == native.TRAVERSAL_AUTO:
+                assert kernels["render_closest"][0] != 0 and kernels["render_any"] == [0] * 5
+        finally:
+            ctx.close()
+    for img, stats in got[1:]:
+        assert img.tobytes() == got[0][0].tobytes() and stats.variance == got[0][1].variance
+
+
+def test_object_placed_twice():
+    """Twins of two objects with one mesh; a third place is no twin."""
+    def place(*shifts):
+        s = soup(1000, 43)
+        s.meshes = s.meshes[1:]
+        m = np.eye(3, 4, dtype=np.float32)
+        objects = []
+        for shift in shifts:
+            m[:, 3] = shift
+            w = np.eye(3, 4, dtype=np.float32)
+            w[:, 3] = -m[:, 3]
+            objects.append(make_object(0, m.ravel().copy(), w.ravel().copy()))
+        s.objects = np.array(objects)
+        s.build_kdtrees(1)
+        return s
+    for shifts, wide in (((0.5, 0.5), False), ((0.5, 2.5), True)):
+        s = place(*shifts)
+        ctx = native.Context(0)
+        try:
+            ctx.upload_scene(s)
+            lo, hi = scenes.scene_box(s)
+            ctx.cast_closest(scenes.random_rays(lo, hi, TIMED_RAYS, 63))
+            assert (ctx.traversal_kernels()["cast"][0] == 0) == wide
+        finally:
+            ctx.close()
+        assert_settled(s, probing_rays(s, 16384, 44))

@@ -83,6 +83,7 @@ struct yar_gpu_ctx {
     yar::Device_Buffer scene_nodes, mesh_nodes, objects, tris;
     yar::Device_Buffer wide_nodes, wide_tris, wide_entries;  // wide_bvh.cuh
     bool wide_planar = false;  // most of the scene's triangles tessellate axis-parallel planes
+    bool wide_twins = false;   // many of the scene's triangles are there twice
     yar::Device_Scene ds;
     yar::Render_Scene render;
 

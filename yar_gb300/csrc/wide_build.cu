@@ -47,6 +47,9 @@ constexpr uint32_t kInnerBit = 0x80000000u;
 
 constexpr uint32_t kPlanarTriangles = 16384;  // of a scene of tessellated planes (yar_gpu_ctx::wide_planar)
 
+// Of a scene of twins (yar_gpu_ctx::wide_twins): one in this many triangles has one.
+constexpr uint32_t kTwinShare = 4;
+
 struct Build_Object {
     uint32_t first;       // of its primitives
     uint32_t tri_offset;  // in the scene's triangle array
@@ -814,6 +817,49 @@ wide_encode_kernel(Pair_Tree tree, const float4* __restrict__ prim_lo, const flo
     }
 }
 
+// ---- twins: triangles with the vertices of another one, in any order (faces
+// modelled twice, an object placed twice).  Twins have one Morton code; those
+// further than kReach places apart among equal codes are not found.
+__device__ __forceinline__ bool same_vertices(const float4* a, const float4* b) {
+    uint32_t found = 0;
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+            if (a[i].x == b[j].x && a[i].y == b[j].y && a[i].z == b[j].z) found |= 1u << i | 8u << j;
+    return found == 63u;
+}
+
+__global__ void __launch_bounds__(kBuildBlock)
+wide_twins_kernel(const float4* __restrict__ prim_lo, const float4* __restrict__ prim_hi, const uint32_t* __restrict__ index,
+                  uint32_t n, const float4* __restrict__ tris, const Build_Object* __restrict__ objects, uint32_t object_count,
+                  uint32_t* twins) {
+    __shared__ float box[6][kBuildBlock + kReach];
+    const uint32_t first = blockIdx.x * kBuildBlock;
+    for (uint32_t k = threadIdx.x; k < kBuildBlock + kReach; k += kBuildBlock)
+        if (first + k < n) {
+            const uint32_t p = index[first + k];
+            const float4 a = prim_lo[p], b = prim_hi[p];
+            box[0][k] = a.x; box[1][k] = a.y; box[2][k] = a.z;
+            box[3][k] = b.x; box[4][k] = b.y; box[5][k] = b.z;
+        }
+    __syncthreads();
+    const uint32_t me = threadIdx.x, i = first + me;
+    bool twin = false;  // of a triangle further on
+    for (uint32_t k = me + 1; k <= me + (uint32_t)kReach && first + k < n && !twin; k++) {
+        bool same = true;
+#pragma unroll
+        for (int c = 0; c < 6; c++) same = same && box[c][k] == box[c][me];
+        if (!same) continue;
+        const uint32_t p = index[i], q = index[first + k];
+        const Build_Object a = objects[object_of(objects, object_count, p)], b = objects[object_of(objects, object_count, q)];
+        twin = a.cx == b.cx && a.cy == b.cy && a.cz == b.cz &&
+               same_vertices(tris + 3 * ((size_t)a.tri_offset + (p - a.first)), tris + 3 * ((size_t)b.tri_offset + (q - b.first)));
+    }
+    const int found = __syncthreads_count(twin);
+    if (threadIdx.x == 0 && found) atomicAdd(twins, (uint32_t)found);
+}
+
 // ---- entries: the deepest kd-tree node whose cell holds a box (a box that
 // ends at a split belongs to the side it lies on), and whether that node is a
 // leaf that holds primitive `prim`
@@ -911,7 +957,7 @@ void wide_release(yar_gpu_ctx* ctx) {
     ctx->ds.wide_entries = nullptr;
     ctx->ds.wide_reach = 0.f;
     ctx->ds.wide_flags = 0u;
-    ctx->wide_planar = false;
+    ctx->wide_planar = ctx->wide_twins = false;
 }
 
 // Scenes without a wide tree (and every cast of theirs) use the kd-tree
@@ -1078,18 +1124,21 @@ cudaError_t wide_build(yar_gpu_ctx* ctx, const yar_flat_scene* scene, const uint
         wide_release(ctx);
         return cudaSuccess;
     }
-    e = cudaMemsetAsync(words, 0, sizeof(uint32_t), st);
+    e = cudaMemsetAsync(words, 0, 2 * sizeof(uint32_t), st);  // triangles of flat nodes, twins
     if (e != cudaSuccess) return e;
+    wide_twins_kernel<<<(totals.valid + kBuildBlock - 1) / kBuildBlock, kBuildBlock, 0, st>>>(
+        prim_lo, prim_hi, index[cur], totals.valid, tris, d_objects, n_objects, words + 1);
     wide_encode_kernel<<<(nodes + 127u) / 128u, 128, 0, st>>>(tree, prim_lo, prim_hi, tris, d_objects, n_objects, children, bases,
                                                               nodes, reach, words, (uint4*)ctx->wide_nodes.ptr, (float4*)ctx->wide_tris.ptr);
     wide_entries_kernel<<<blocks, kBuildBlock, 0, st>>>(tris, (const uint2*)ctx->mesh_nodes.ptr, (const uint2*)ctx->scene_nodes.ptr,
                                                         d_objects, n_objects, prims, (float4*)ctx->wide_entries.ptr);
     e = cudaGetLastError();
-    uint32_t flat = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&flat, words, sizeof(flat), cudaMemcpyDeviceToHost, st);
+    uint32_t found[2] = {0u, 0u};
+    if (e == cudaSuccess) e = cudaMemcpyAsync(found, words, sizeof(found), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return e;
-    ctx->wide_planar = flat >= kPlanarTriangles && flat > totals.valid / 2u;
+    ctx->wide_planar = found[0] >= kPlanarTriangles && found[0] > totals.valid / 2u;
+    ctx->wide_twins = 2ull * found[1] * kTwinShare > totals.valid;  // (of two, one was counted)
     ctx->ds.wide_entries = (const float4*)ctx->wide_entries.ptr;
     ctx->ds.wide_nodes = (const uint4*)ctx->wide_nodes.ptr;
     ctx->ds.wide_tris = (const float4*)ctx->wide_tris.ptr;
