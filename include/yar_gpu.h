@@ -385,13 +385,16 @@ typedef struct yar_gpu_options {
  * settle walk the kd-tree one per thread (renders of scenes of tessellated
  * axis-parallel planes walk it for every ray, as PER_RAY).
  * The others, fixed by the options or chosen for scenes without such a tree
- * (a rotated or scaled object leaves it out), walk the kd-tree: persistent warps
+ * (a rotated or scaled object leaves it out) and for rays that it does not
+ * suit (closest hits in a scene where many triangles are there twice, casts of
+ * a batch of which a quarter did not settle, as from origins beyond 64 times the
+ * scene's size, and those after it), walk the kd-tree: persistent warps
  * at high occupancy (PERSISTENT_64: a register cap for 8 blocks of 128
  * threads per SM, 64 registers, for closest-hit rays and for 12 blocks, 40
  * registers, for any-hit rays), persistent warps with up to 128 registers
- * (PERSISTENT_128), or one ray per thread.  In those scenes AUTO times, on the
- * first large enough batch of each ray kind (and each render bounce) after the
- * scene upload, all of them and keeps the fastest. */
+ * (PERSISTENT_128), or one ray per thread.  AUTO times them on the first large
+ * enough batch of each ray kind (and each render bounce) and keeps the fastest
+ * for the uploaded scene. */
 #define YAR_TRAVERSAL_AUTO 0
 #define YAR_TRAVERSAL_PERSISTENT_64 1
 #define YAR_TRAVERSAL_PERSISTENT_128 2

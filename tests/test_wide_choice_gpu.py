@@ -224,3 +224,38 @@ def test_object_placed_twice():
         finally:
             ctx.close()
         assert_settled(s, probing_rays(s, 16384, 44))
+
+
+def test_rays_from_far_away():
+    """Rays from origins that the tree's margins do not cover walk the kd-tree;
+    after a batch of them the casts are timed among the kd-tree kernels.  Small
+    batches and nearer ones change nothing."""
+    s = soup(5000, 51)
+    lo, hi = scenes.scene_box(s)
+    rays = scenes.random_rays(lo, hi, TIMED_RAYS, 64)
+    far = rays.copy()
+    far[:, 0:3] -= np.float32(1000) * far[:, 4:7]
+    some = rays.copy()
+    some[::6] = far[::6]
+    want = native.Context(0, traversal_kernel=native.TRAVERSAL_PER_RAY)
+    ctx = native.Context(0)
+    try:
+        for c in (ctx, want):
+            c.upload_scene(s)
+        for batch, n, kernels in ((rays, TIMED_RAYS, (True, True)), (some, TIMED_RAYS, (True, True)),
+                                  (far, 60000, (True, True)), (far, TIMED_RAYS, (True, True)),
+                                  (far, TIMED_RAYS, (False, True)), (rays, TIMED_RAYS, (False, True))):
+            got, ref = ctx.cast_closest(batch[:n]), want.cast_closest(batch[:n])
+            for g, w in zip(got, ref):
+                assert g.tobytes() == w.tobytes()
+            assert tuple(k == 0 for k in ctx.traversal_kernels()["cast"]) == kernels
+        for batch in (far, far):
+            assert ctx.cast_any(batch).tobytes() == want.cast_any(batch).tobytes()
+        assert 0 not in ctx.traversal_kernels()["cast"]
+        ctx.upload_scene(s)
+        assert ctx.traversal_kernels()["cast"] == [0, 0]
+        ctx.cast_closest(rays)
+        assert ctx.traversal_kernels()["cast"] == [0, 0]
+    finally:
+        ctx.close()
+        want.close()

@@ -180,8 +180,8 @@ extern "C" int yar_gpu_create(yar_gpu_ctx** out, const yar_gpu_options* options)
     }
     e = cudaSetDevice(ctx->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_error, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(ctx->d_error, 0, sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_error, 2 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(ctx->d_error, 0, 2 * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_counter, yar_gpu_ctx::kPipeChunks * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev_start);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev_stop);
@@ -402,14 +402,26 @@ int ensure_staging(yar_gpu_ctx* ctx, uint32_t n, bool closest) {
     return YAR_OK;
 }
 
-int check_error_word(yar_gpu_ctx* ctx) {
-    int h = 0;
+// The end of a cast of n rays (closest or any hit).
+// A ray that the wide tree leaves to the kd-tree walks it alone, one per thread,
+// which in a deep tree takes twice the time of the kernel that timing picks:
+// 4.2M closest-hit rays from 100 times the size of 2.4M triangles (which the
+// tree's margins do not cover) 15.1 ms against 7.1, any hits 6.1 against 4.0.
+// Once a quarter of a larger batch did (nearer rays: 1%), this kind's casts of
+// the scene are timed among the kd-tree kernels.
+int finish_cast(yar_gpu_ctx* ctx, uint32_t n, bool closest) {
+    constexpr uint32_t kLargeBatch = 1u << 16, kWalkShare = 4;
+    int h[2] = {0, 0};
     int* word = reinterpret_cast<int*>(pinned_block(ctx));
-    if (!word) word = &h;
-    cudaError_t e = cudaMemcpyAsync(word, ctx->d_error, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
+    if (!word) word = h;
+    cudaError_t e = cudaMemcpyAsync(word, ctx->d_error, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "kernel");
-    if (*word) {
+    const uint32_t walked = (uint32_t)word[1] - ctx->walked;
+    ctx->walked = (uint32_t)word[1];
+    int& kernel = ctx->cast_kernel[closest ? 0 : 1];
+    if (kernel == kCastWide && n >= kLargeBatch && walked > n / kWalkShare) kernel = -1;
+    if (word[0]) {
         cudaMemsetAsync(ctx->d_error, 0, sizeof(int), ctx->stream);
         return fail(ctx, YAR_ERR_CAPACITY, "kd-tree traversal stack overflow");
     }
@@ -493,6 +505,7 @@ int cast_pipelined(yar_gpu_ctx* ctx, const yar_ray* rays, uint32_t n, const yar_
             a.occluded = (uint8_t*)ctx->d_occ.ptr + first;
         }
         a.answers = (uint32_t*)ctx->d_answers.ptr + first;
+        a.walked = (uint32_t*)ctx->d_error + 1;
         e = closest ? launch_extend(ctx->ds, a, kernel, ks) : launch_shadow(ctx->ds, a, kernel, ks);
         if (e == cudaSuccess) e = cudaEventRecord(ctx->pipe_cast_done[c], ks);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->pipe_out, ctx->pipe_cast_done[c], 0);
@@ -516,7 +529,7 @@ int cast_pipelined(yar_gpu_ctx* ctx, const yar_ray* rays, uint32_t n, const yar_
         if (e == cudaSuccess) e = e2;
     }
     if (e != cudaSuccess) return cuda_fail(ctx, e, "pipelined cast");
-    return check_error_word(ctx);
+    return finish_cast(ctx, n, closest);
 }
 
 int cast(yar_gpu_ctx* ctx, const yar_ray* rays, uint32_t n, const yar_hit_soa* hits, uint8_t* occluded,
@@ -614,6 +627,7 @@ int cast(yar_gpu_ctx* ctx, const yar_ray* rays, uint32_t n, const yar_hit_soa* h
     a.bary = d_bary;
     a.occluded = d_occ;
     a.answers = (uint32_t*)ctx->d_answers.ptr;
+    a.walked = (uint32_t*)ctx->d_error + 1;
     int& kernel = ctx->cast_kernel[closest ? 0 : 1];
     if (kernel < 0 && n >= kTuneMinRays) {
         e = tune_cast(ctx->ds, a, !closest, ctx->stream, ctx->ev_start, ctx->ev_stop, &kernel);
@@ -638,7 +652,7 @@ int cast(yar_gpu_ctx* ctx, const yar_ray* rays, uint32_t n, const yar_hit_soa* h
         }
         if (e != cudaSuccess) return cuda_fail(ctx, e, "result download");
     }
-    int rc = check_error_word(ctx);
+    int rc = finish_cast(ctx, n, closest);
     if (small && rc != YAR_ERR_CUDA) {
         if (d_t) memcpy(hits->t, d_t, (size_t)n * 4);
         if (d_prim) memcpy(hits->prim, d_prim, (size_t)n * 4);

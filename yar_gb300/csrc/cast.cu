@@ -332,7 +332,7 @@ settle_wide(const __grid_constant__ Device_Scene s, const __grid_constant__ Cast
             if ((uint32_t)lane < k) {
                 const uint2 entry = list[listed + lane];
                 Hit h;
-                const int status = wide_settle<ANY>(s, a.rays, entry.x, entry.y, h);
+                const int status = wide_settle<ANY>(s, a.rays, entry.x, entry.y, a.walked, h);
                 write_settled<ANY>(status, h, entry.x, a);
             }
             __syncwarp();

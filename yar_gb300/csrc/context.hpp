@@ -93,7 +93,10 @@ struct yar_gpu_ctx {
     yar::Device_Buffer d_answers;  // the wide tree's answers of a cast
     // page-locked host block for what small synchronous calls move (pinned_block)
     char* pinned = nullptr;
-    int* d_error = nullptr;  // device error word (stack overflow, bounded-wait expiry)
+    // device words: error (stack overflow, bounded-wait expiry); rays of casts that
+    // the wide tree left to a walk of the kd-tree, added up (walked: as last read)
+    int* d_error = nullptr;
+    uint32_t walked = 0;
     uint32_t* d_counter = nullptr;  // ray hand-out counters of the persistent cast kernels, one per pipeline chunk
     // host-buffer casts in chunks: copies in, the traversal on two compute
     // streams (the context's and pipe_compute) and copies out overlap
@@ -181,6 +184,7 @@ struct Cast_Args {
     uint8_t* occluded = nullptr;
     // the wide tree's answers, one word per ray position (kCastWide)
     uint32_t* answers = nullptr;
+    uint32_t* walked = nullptr;       // adds up the rays that walk the kd-tree (kCastWide)
 };
 // Traversal kernels: persistent warps at high occupancy (closest hit 10
 // blocks per SM, any hit 12 blocks), persistent

@@ -399,9 +399,14 @@ __device__ __forceinline__ bool entry_interval(float4 lo, float4 hi, float3 o, f
     return true;
 }
 
-// The kd-tree's walk of one ray, for rays that the wide tree does not settle.
+// The kd-tree's walk of one ray, for rays that the wide tree does not settle
+// (added to *walked, if given).
 template <bool ANY>
-__device__ __noinline__ int kd_walk(const Device_Scene& s, const float4* rays, uint32_t ray, Hit& hit) {
+__device__ __noinline__ int kd_walk(const Device_Scene& s, const float4* rays, uint32_t ray, uint32_t* walked, Hit& hit) {
+    if (walked) {
+        const unsigned here = __activemask();
+        if ((int)(threadIdx.x & 31u) == __ffs((int)here) - 1) atomicAdd(walked, (uint32_t)__popc(here));
+    }
     const float4 r0 = __ldg(rays + 2 * (size_t)ray), r1 = __ldg(rays + 2 * (size_t)ray + 1);
     Traversal<ANY> tr;
     Local_Stack stack;
@@ -417,7 +422,8 @@ __device__ __noinline__ int kd_walk(const Device_Scene& s, const float4* rays, u
 // and hit that the kd-tree gives.  A miss (kWideNone) needs no settling.
 
 template <bool ANY>
-__device__ __forceinline__ int wide_settle(const Device_Scene& s, const float4* rays, uint32_t ray, uint32_t answer, Hit& hit) {
+__device__ __forceinline__ int wide_settle(const Device_Scene& s, const float4* rays, uint32_t ray, uint32_t answer,
+                                           uint32_t* walked, Hit& hit) {
     if (!(answer & kWideTie)) {
         const float4 r0 = __ldg(rays + 2 * (size_t)ray), r1 = __ldg(rays + 2 * (size_t)ray + 1);
         const float4* p = s.wide_tris + 4 * (size_t)answer;
@@ -474,7 +480,7 @@ __device__ __forceinline__ int wide_settle(const Device_Scene& s, const float4* 
         }
         if (visited) return 1;
     }
-    return kd_walk<ANY>(s, rays, ray, hit);
+    return kd_walk<ANY>(s, rays, ray, walked, hit);
 }
 
 } // namespace yar
