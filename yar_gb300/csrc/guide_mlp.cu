@@ -521,6 +521,8 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_kernel(Mlp_Args a) {
                 parity ^= 1u;
             }
         }
+        if (!ok && issuer) drain(base + kTrMisc + 128);
+        __syncwarp();
     } else {
         const uint32_t ready = base + kTrMisc + 16 * group, done = ready + 8;
         const uint32_t lane_addr = tmem + 64u * group + ((uint32_t)(tid & ~31) << 16);
@@ -567,12 +569,14 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_kernel(Mlp_Args a) {
             }
         }
     }
-    // (a group may give up on a step that the issuing warp has issued as its last)
+    const bool drained = !ok;
     ok = !__syncthreads_or(!ok);
     tc::fence_after_sync();
-    if (!ok && threadIdx.x == 0) atomicOr(a.err, 2);
-    if (!ok && group == kTrGroups && tid == 0) drain(base + kTrMisc + 128);
-    __syncwarp();
+    if (!ok) {
+        if (threadIdx.x == 0) atomicOr(a.err, 2);
+        // a group gave up on a step that the issuing warp had issued as its last
+        if (threadIdx.x == kTrGroups * kRows && !drained) drain(base + kTrMisc + 128);
+    }
 
     // partial gradients of this CTA, in the parameter layout [out][in]
     float* part = a.partials + (size_t)blockIdx.x * kGuideParams;
