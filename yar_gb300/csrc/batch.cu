@@ -14,9 +14,9 @@
 // of large ones and finish early.  A one-thread kernel stamps the GPU clock when each scene's
 // film is resolved: per-scene completion times come from the device.
 //
-// Autotuner: before capture, (1) the traversal kernel of each scene that has
-// no wide tree and no fixed kernel is chosen by timing the kd-tree kernels on
-// 2^16 random rays in its box (tune_cast), and
+// Autotuner: before capture, (1) the traversal kernels of each scene that the
+// options do not fix and the wide tree does not cast are chosen by timing the
+// kd-tree kernels on 2^16 random rays in its box (tune_cast), and
 // (2) the branch count and the chunk capacity (paths in flight per branch)
 // are chosen by capturing and timing the whole batch at one sample per pixel
 // for each candidate; the full-sample graph is then captured with the winner.

@@ -354,8 +354,8 @@ extern "C" int yar_gpu_upload_scene(yar_gpu_ctx* ctx, const yar_flat_scene* scen
     // any hit 3.2 against 11.2), but renders of a scene of tessellated planes
     // walk the kd-tree, one ray per thread: the render's rays reach a plane
     // together, and there a binary descent takes fewer instructions than eight
-    // boxes a level (the GGX room at 512 x 512, 64 samples: 42.4 ms against
-    // 43.1 ms; equal at 3,200 triangles a wall).
+    // boxes a level (the GGX room at 512 x 512, 64 samples: 34.9 ms against
+    // 36.6 ms, its guided form 36.0 against 39.4; equal at 3,200 triangles a wall).
     int fixed = ctx->forced_kernel;
     if (fixed < 0) {
         e = wide_build(ctx, scene, tri_offset.data(), node_offset.data());
@@ -379,7 +379,9 @@ extern "C" int yar_gpu_upload_scene(yar_gpu_ctx* ctx, const yar_flat_scene* scen
         ctx->cast_kernel[k] = fixed == kCastWide ? wide : fixed;
         for (int& b : ctx->render_kernel[k]) b = fixed != kCastWide ? fixed : ctx->wide_planar ? (int)kCastPerRay : wide;
     }
-    ctx->render_tuned = ctx->forced_kernel >= 0;  // the first render of a scene reads its queue lengths on the host
+    // the first render of a scene drives its bounces from the host, whose queue
+    // lengths the timing of the kd-tree kernels takes (also where nothing is timed)
+    ctx->render_tuned = ctx->forced_kernel >= 0;
     memset(ctx->render_tune_ms, 0, sizeof(ctx->render_tune_ms));
     memset(ctx->render_tune_queues, 0, sizeof(ctx->render_tune_queues));
     ctx->has_scene = true;

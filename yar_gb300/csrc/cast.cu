@@ -185,9 +185,9 @@ __global__ void __launch_bounds__(kCastBlock) cast_per_ray_vote(Device_Scene s, 
 // node, test a leaf child) per warp iteration.  Lanes whose ray is done wait
 // until kWideRefill of them are, then write their results (a miss is final, a
 // hit leaves its answer for the second kernel) and take new rays.  Bound by
-// issue (78% of the cycles on 16M random rays in 2.4M triangles, 17 of 32 lanes
-// in an instruction, about 200 warp instructions per ray against the kd-tree
-// kernel's 880); measured there, closest / any hit: 8 blocks of 128 threads per
+// issue (76% of the cycles on 4.2M random rays in 2.4M triangles, 17 of 32 lanes
+// in an instruction, 193 warp instructions per ray against the kd-tree
+// kernel's 880); measured with 16M, closest / any hit: 8 blocks of 128 threads per
 // SM 4.4 / 3.2 ms, 6 blocks 4.6 / 3.5; refills at 4, 8, 12, 16, 20 done lanes
 // 5.1, 4.81, 4.78, 5.2, 5.5 ms (before the entries below); tests as soon as
 // half as many lanes wait for one as visit 4.8 ms, when more do 5.0.
@@ -195,8 +195,8 @@ __global__ void __launch_bounds__(kCastBlock) cast_per_ray_vote(Device_Scene s, 
 // settle_wide: every hit against the kd-tree, with full warps.  A settled hit
 // costs dependent loads; inside the first kernel (at its registers, with the
 // lanes that happen to be done) they took as long as the traversal: 7.9 ms
-// together, 5.7 as two kernels, 4.4 once the descents begin at the triangles'
-// entries.  Now bound by scattered DRAM reads (about 4 TB/s).
+// together, 5.7 as two kernels, 4.3 once the descents begin at the triangles'
+// entries.  Now bound by scattered DRAM accesses (3.1 TB/s).
 constexpr int kWideShortStack = 10;  // shared-memory entries; deeper ones in local memory
 constexpr int kWideRefill = 12;
 constexpr int kWideBlocks = 8, kSettleBlocks = 8;

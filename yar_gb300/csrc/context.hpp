@@ -156,7 +156,7 @@ char* pinned_block(yar_gpu_ctx* ctx);
 int device_alloc(yar_gpu_ctx* ctx, Device_Buffer& b, size_t bytes);
 void device_free(Device_Buffer& b);
 // A call's working memory: as device_alloc, but where there is none the scene's
-// wide tree (about 0.3 KB a triangle) makes room and its casts walk the kd-tree
+// wide tree (about 0.2 KB a triangle) makes room and its casts walk the kd-tree
 // from then on.  Called before the call looks up its traversal kernels.
 int work_alloc(yar_gpu_ctx* ctx, Device_Buffer& b, size_t bytes);
 // Frees the wide tree of the scene; false without one.

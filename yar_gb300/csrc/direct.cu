@@ -23,7 +23,7 @@
 //
 // The rays bound it: 10 per sample and a few hundred instructions for each.
 // The Cornell box with a quad light of 4 samples, two delta lights and a spot,
-// 512 x 512 samples of 16: 6.0 ms, of which the casts and their settling take
+// 512 x 512 samples of 16: 5.7 ms, of which the casts and their settling take
 // 40%, the light and BSDF samples 35%.  One kernel that walked through a
 // sample's units and traced their rays inline through the kd-tree took 25 ms
 // (28 ms in all): at 230 registers 12% of the warps were resident, and lanes

@@ -55,9 +55,9 @@ __device__ __forceinline__ float clamp1(float x) { return x < -1.f ? -1.f : (x >
 // multiples of pi/2 (three-part constant, Cody and Waite), Taylor polynomials
 // whose first four steps are two-float products (Dekker; the products' errors by
 // FMA), about 2^-44 relative.  Where the float nearest to the sum is not the
-// same 2^-38 to either side (one argument in 8,000), or outside [-7, 7], the
-// FP64 functions decide, so the results are theirs: compared over every float
-// in [-7, 7].
+// same 2^-38 to either side (one in 8,000 of angles drawn evenly; all below
+// 2^-32), or outside [-7, 7], the FP64 functions decide, so the results are
+// theirs: compared over every float in [-8, 8].
 struct Two_Float {
     float h, l;
 };

@@ -1351,8 +1351,9 @@ __device__ __forceinline__ V3 sphere_sampler_sample(const Sphere_Sampler& ss, fl
 // dependent load after another, so resident warps count more than spills: the
 // bump-mapped box took 38.9 ms at 4 blocks, 36.2 at 5, 32.5 at 8 (1.4 KB of
 // spills); delta materials with textures 28.2, 27.8 and 26.2 ms, a small image
-// of them (333 x 250) 5.40, 5.42 and 5.49 ms.  With the texture code in
+// of them (333 x 251) 5.40, 5.42 and 5.49 ms.  With the texture code in
 // kShadeFull at 3 blocks: 39.2, 28.4 and 5.56 ms, and 6.91 ms for the lights.
+// (Its guided form takes the same bound and was not measured apart.)
 enum Shade_Kind { kShadePlain, kShadeFull, kShadeTextured };
 constexpr int kShadeBlocks[3] = {4, 3, 8};
 template <bool GUIDED, int KIND>
@@ -2009,7 +2010,7 @@ __device__ __forceinline__ void key_group(uint32_t key, uint32_t& rank, int& lea
 
 // Both kernels below are bound by the queue's bytes (9 and 5 B per entry) once
 // their atomics on the few class counters are few: one per class and block
-// here, one per class and kOrderItems entries there.  Over a render of 2.4M
+// here, one per class and kOrderItems entries there.  Over a render of 4.1M
 // triangles at 1080p (76 bounces of two chunks) they took 2.0 ms each with one
 // atomic per class and warp (a million on four words for the first bounce),
 // 0.44 and 0.60 ms as below.
